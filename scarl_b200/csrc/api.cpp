@@ -136,6 +136,11 @@ class HostPool {
 constexpr int kRingSlots = 4;
 constexpr size_t kRingChunk = (size_t)32 << 20;
 constexpr size_t kRingMin = (size_t)8 << 20;
+// literal DCT tiles generated and held together up to this many bytes: few
+// launches over all of them, the tiles staying in L2 for the gather (8 tiles of
+// 23^3: 45 us a sample against 250 us tile by tile); larger samples fill the
+// GPU with one tile and save the tiles' round trip through memory
+constexpr size_t kDctBatch = (size_t)64 << 20;
 
 }  // namespace
 
@@ -163,7 +168,7 @@ struct scarl_ctx {
   HostPool* hpool = nullptr;
   std::map<std::string, PaddedPlan> plans;
   std::map<long long, Buf> twiddles;
-  std::map<int, Buf> dct_tabs;
+  std::map<std::pair<int, int>, Buf> dct_tabs;  // (length, inputs) -> folded cosines
   bool profile = false;
   long long launches = 0;
   unsigned long long h2d = 0, d2h = 0;
@@ -1282,79 +1287,92 @@ int upload_blend_tables(scarl_ctx* ctx, const scarl_layout& lay, int partitionTy
   return SCARL_OK;
 }
 
-int dct_table(scarl_ctx* ctx, int N, const double** out) {
-  auto it = ctx->dct_tabs.find(N);
+// Folded cosine matrix of a DCT-III of length N over K inputs, kept by the context.
+int dct_table(scarl_ctx* ctx, int N, int K, const double** out) {
+  const std::pair<int, int> key(N, K);
+  auto it = ctx->dct_tabs.find(key);
   if (it != ctx->dct_tabs.end()) {
     *out = (const double*)it->second.p;
     return SCARL_OK;
   }
-  Buf b;
-  RC(ensure(ctx, b, (size_t)4 * N * 8));
+  Buf raw, b;
+  RC(ensure(ctx, raw, (size_t)4 * N * 8));
   std::vector<double> c(4 * (size_t)N);
   for (int m = 0; m < 4 * N; ++m) c[m] = std::cos(M_PI * (double)m / (2.0 * (double)N));
-  CK(cudaMemcpy(b.p, c.data(), c.size() * 8, cudaMemcpyHostToDevice));
-  ctx->dct_tabs[N] = b;
+  int rc = ensure(ctx, b, (size_t)K * round_up((N + 1) / 2, 2) * 8);
+  if (rc == SCARL_OK && (cudaMemcpy(raw.p, c.data(), c.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+                         launch_dct_table((const double*)raw.p, N, K, (double*)b.p, ctx->stream) != cudaSuccess ||
+                         cudaStreamSynchronize(ctx->stream) != cudaSuccess))
+    rc = fail(ctx, SCARL_EDEVICE, std::string("cosine table: ") + cudaGetErrorString(cudaGetLastError()));
+  release(ctx, raw);
+  if (rc != SCARL_OK) {
+    release(ctx, b);
+    return rc;
+  }
+  ctx->dct_tabs[key] = b;
   *out = (const double*)b.p;
   return SCARL_OK;
 }
 
-// gen_std_gauss_FFT on the device into dev_out (Np doubles).
+// gen_std_gauss_FFT of nt tiles on the device; tile t spans xRange[3 t ..],
+// draws with key + t and leaves through the output stage epi (nt > 1: plain
+// tiles one after the other).
 // full_z: the spectrum spans every kz (gen_Std_Gauss_FFT_MPI,
 // SRC_F/fftw_ScaRL.f90:469-476), else the (Np/2)^3 octant.
-int dct_tile(scarl_ctx* ctx, double* dev_out, const int Np[3], const double xRange[3],
-             const double corrL[3], const double* phi_dev, const double* gamma_dev,
-             uint32_t key, bool full_z = false) {
+int dct_tiles(scarl_ctx* ctx, int nt, const int Np[3], const double* xRange, const double corrL[3],
+              const double* phi_dev, const double* gamma_dev, uint32_t key, bool full_z, const Epilogue& epi) {
   DctArgs a;
   std::memset(&a, 0, sizeof a);
-  size_t ktot = 1, t1n, t2n;
-  std::vector<double> ex;
+  size_t nexp = 0;
   for (int d = 0; d < 3; ++d) {
     a.Np[d] = Np[d];
     a.K[d] = (full_z && d == 2) ? Np[d] : Np[d] / 2;
     a.corrL[d] = corrL[d];
-    ktot *= (size_t)a.K[d];
+    nexp += (size_t)a.K[d];
   }
-  t1n = (size_t)Np[0] * a.K[1] * a.K[2];
-  t2n = (size_t)Np[0] * Np[1] * a.K[2];
+  for (int d = 0; d < 3; ++d) RC(dct_table(ctx, Np[d], a.K[d], &a.tab[d]));
+  int64_t nsk, n1, n2;
+  dct_sizes(a.Np, a.K, &nsk, &n1, &n2);
+  RC(ensure(ctx, ctx->sk, (size_t)nsk * nt * 8));
+  RC(ensure(ctx, ctx->t1, (size_t)n1 * nt * 8));
+  RC(ensure(ctx, ctx->t2, (size_t)n2 * nt * 8));
+  RC(ensure(ctx, ctx->dtabs, nexp * nt * 8));
   // per-axis exp(-PI k^2) factors, SRC_F/fftw_ScaRL.f90:300-326
-  std::vector<double> h;
-  size_t off[3];
-  for (int d = 0; d < 3; ++d) {
-    off[d] = h.size();
-    const double delta_x = xRange[d] / (double)(Np[d] - 1);
-    const double k_max = 1.0 / delta_x;
-    const double dk = k_max / (double)(Np[d] - 1);
-    for (int i = 0; i < a.K[d]; ++i) {
-      const double kp = (double)i * dk / corrL[d];
-      h.push_back(std::exp(-kPiRef * (kp * kp)));
-    }
-  }
-  h.push_back(0.0);
   void* hp;
-  RC(pinned(ctx, h.size() * 8, &hp));
-  std::memcpy(hp, h.data(), h.size() * 8);
-  RC(ensure(ctx, ctx->dtabs, h.size() * 8));
-  RC(upload_pinned(ctx, ctx->dtabs.p, h.size() * 8));
-  const double* dt = (const double*)ctx->dtabs.p;
-  a.cx = dt + off[0];
-  a.cy = dt + off[1];
-  a.cz = dt + off[2];
-  RC(ensure(ctx, ctx->sk, std::max<size_t>(ktot, 1) * 8));
-  RC(ensure(ctx, ctx->t1, std::max<size_t>(t1n, 1) * 8));
-  RC(ensure(ctx, ctx->t2, std::max<size_t>(t2n, 1) * 8));
+  RC(pinned(ctx, nexp * nt * 8, &hp));
+  double* h = (double*)hp;
+  for (int t = 0; t < nt; ++t)
+    for (int d = 0; d < 3; ++d) {
+      const double delta_x = xRange[3 * t + d] / (double)(Np[d] - 1);
+      const double k_max = 1.0 / delta_x;
+      const double dk = k_max / (double)(Np[d] - 1);
+      for (int i = 0; i < a.K[d]; ++i) {
+        const double kp = (double)i * dk / corrL[d];
+        *h++ = std::exp(-kPiRef * (kp * kp));
+      }
+    }
+  RC(upload_pinned(ctx, ctx->dtabs.p, nexp * nt * 8));
+  a.nt = nt;
+  a.cexp = (const double*)ctx->dtabs.p;
   a.sk = (double*)ctx->sk.p;
   a.t1 = (double*)ctx->t1.p;
   a.t2 = (double*)ctx->t2.p;
-  a.out = dev_out;
   a.phi = phi_dev;
   a.gamma = gamma_dev;
   a.k0 = key;
-  a.k1 = 0;
-  a.stream = 0;
-  for (int d = 0; d < 3; ++d) RC(dct_table(ctx, Np[d], &a.ctab[d]));
+  a.epi = epi;
   Prof p(ctx, "k_dct_literal", 4);
   CK(launch_dct_literal(a, ctx->stream));
   return SCARL_OK;
+}
+
+// One tile without blending into dev_out (Np doubles).
+int dct_tile(scarl_ctx* ctx, double* dev_out, const int Np[3], const double xRange[3], const double corrL[3],
+             const double* phi_dev, const double* gamma_dev, uint32_t key, bool full_z = false) {
+  Epilogue epi;
+  std::memset(&epi, 0, sizeof epi);
+  epi.out = dev_out;
+  return dct_tiles(ctx, 1, Np, xRange, corrL, phi_dev, gamma_dev, key, full_z, epi);
 }
 
 // Literal Shino GenArgs for one tile (SRC_F/fftw_ScaRL.f90:157-255).
@@ -2753,8 +2771,12 @@ int scarl_generate_sample(scarl_ctx* ctx, const scarl_sample* s, const scarl_gen
   if (gen == SCARL_GEN_DCT) {
     for (int d = 0; d < 3; ++d)
       if (lay.Np[d] < 2) return fail(ctx, SCARL_EINVAL, "Np must be >= 2");
-    RC(ensure(ctx, ctx->tile, ntile * 8));
   }
+  // literal tiles that fit kDctBatch bytes together: one launch per step over
+  // all of them, then one gather of the blended field; larger ones one after
+  // the other, each blended by its z transform's output stage
+  const bool dct_batch = gen == SCARL_GEN_DCT && lay.nb_tiles > 1 && ntile * 8 * lay.nb_tiles <= kDctBatch &&
+                         ensure(ctx, ctx->tile, ntile * 8 * lay.nb_tiles) == SCARL_OK;
   const void* phi_all = nullptr;
   if (gen == SCARL_GEN_DCT && o.phiK)
     RC(in_dev(ctx, ctx->stage_in, o.phiK, nk * lay.nb_tiles * 8, &phi_all));
@@ -2877,10 +2899,40 @@ int scarl_generate_sample(scarl_ctx* ctx, const scarl_sample* s, const scarl_gen
         RC(run_passes(ctx, 8, a));
       } else {
         const double* phi = phi_all ? (const double*)phi_all + nk * r : nullptr;
-        RC(dct_tile(ctx, (double*)ctx->tile.p, lay.Np, t.xRange, s->corrL, phi, nullptr, (uint32_t)seedStart,
-                    gm == SCARL_FFT_MPI));
-        Prof p(ctx, "k_blend_tile");
-        CK(launch_blend_tile(8, ctx->tile.p, lay.Np, e, ctx->stream));
+        if (!dct_batch) {
+          RC(dct_tiles(ctx, 1, lay.Np, t.xRange, s->corrL, phi, nullptr, (uint32_t)seedStart, gm == SCARL_FFT_MPI, e));
+        } else if (r == 0) {
+          std::vector<double> xr((size_t)3 * lay.nb_tiles);
+          for (int q = 0; q < lay.nb_tiles; ++q) {
+            scarl_tile tq;
+            tile_geometry(&lay, s->xMinGlob, q, &tq);
+            std::memcpy(&xr[3 * (size_t)q], tq.xRange, sizeof tq.xRange);
+          }
+          Epilogue plain;
+          std::memset(&plain, 0, sizeof plain);
+          plain.out = ctx->tile.p;
+          RC(dct_tiles(ctx, lay.nb_tiles, lay.Np, xr.data(), s->corrL, phi, nullptr, (uint32_t)seedStart, false, plain));
+          BlendGather g;
+          std::memset(&g, 0, sizeof g);
+          g.tiles = (const double*)ctx->tile.p;
+          g.out = (double*)dev;
+          for (int d = 0; d < 3; ++d) {
+            g.Np[d] = lay.Np[d];
+            g.No[d] = lay.Np_ovlp[d];
+            g.T[d] = lay.topo_shape[d];
+            g.L[d] = lay.L[d];
+            g.sw[d] = axes[d].sw64;
+            g.fl[d] = axes[d].flags;
+          }
+          g.sws = axes[3].sw64 - axes[0].sw64;  // the tiles' tables lie one after the other
+          g.fls = axes[3].flags - axes[0].flags;
+          g.pou = epi.apply_pou;
+          g.marginal = epi.marginal;
+          g.ms = ms;
+          g.mu = mmu;
+          Prof p(ctx, "k_blend_gather");
+          CK(launch_blend_gather(g, ctx->stream));
+        }
       }
       if ((stream_out || ring_out) && t.topo_pos[0] == lay.topo_shape[0] - 1) {
         const int ty = t.topo_pos[1], tz = t.topo_pos[2];

@@ -1,7 +1,5 @@
 // post.cu -- standalone post steps of the localization method, each a
 // memory-bound elementwise or gather pass over HBM:
-//   k_blend_tile   : one tile into the global field (PoU, overlap sum,
-//                    assembly, marginal) -- the DCT path's epilogue;
 //   k_apply_pou    : apply_UnityPartition_mtx (SRC_F/main_ScaRL.f90:1216-1301);
 //   k_add_overlap  : add_overlap over all tiles held in HBM (:984-1210);
 //   k_marginal     : multiVariateTransformation (:1355-1395);
@@ -17,26 +15,6 @@ namespace scarl {
 static inline unsigned grid_for(int64_t n, int threads, int cap = 148 * 32) {
   int64_t g = (n + threads - 1) / threads;
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(g, cap));
-}
-
-template <typename T>
-__global__ void k_blend_tile(const T* __restrict__ tile, int Nx, int Ny, int Nz, const Epilogue e) {
-  const int64_t n = (int64_t)Nx * Ny * Nz;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(i % Nx);
-    const int64_t r = i / Nx;
-    const int y = (int)(r % Ny), z = (int)(r / Ny);
-    epilogue_point<T>(e, x, y, z, Nx, Ny, tile[i]);
-  }
-}
-
-cudaError_t launch_blend_tile(int dt, const void* tile, const int Np[3], const Epilogue& e,
-                              cudaStream_t s) {
-  const int64_t n = (int64_t)Np[0] * Np[1] * Np[2];
-  if (dt == 8) k_blend_tile<double><<<grid_for(n, 256), 256, 0, s>>>((const double*)tile, Np[0], Np[1], Np[2], e);
-  else k_blend_tile<float><<<grid_for(n, 256), 256, 0, s>>>((const float*)tile, Np[0], Np[1], Np[2], e);
-  return cudaGetLastError();
 }
 
 struct PouAxes { BlendAxis ax[3]; };

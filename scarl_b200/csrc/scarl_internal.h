@@ -142,28 +142,45 @@ cudaError_t launch_spectrum_sum(const GenArgs& a, const double* rx, const double
                                 cudaStream_t s);
 int spectrum_sum_blocks();
 
-// Literal DCT-III path (FP64).
+// Literal DCT-III path (FP64): nt tiles of one shape in one launch per step.
 struct DctArgs {
   int Np[3];
   int K[3];
-  const double* cx;  // per-axis corrL * exp(-PI k^2) factors, order of the reference
-  const double* cy;
-  const double* cz;
+  int nt;
+  const double* cexp;   // per tile: exp(-PI k_d^2), K0 + K1 + K2 values
   double corrL[3];
-  const double* phi;    // injected phases (K0*K1*K2) or null (Philox uniforms)
+  const double* phi;    // injected phases (nt x K0*K1*K2) or null (Philox uniforms)
   const double* gamma;  // injected amplitudes or null (1)
-  uint32_t k0, k1, stream;
-  double* sk;           // K0*K1*K2 spectrum
-  double* t1;           // N0*K1*K2
-  double* t2;           // N0*N1*K2
-  double* out;          // N0*N1*N2
-  const double* ctab[3];  // 2*cos(pi m / (2 N)) (and 1 at i = 0), m < 4N
+  uint32_t k0, k1, stream;  // tile t draws with key (k0 + t, k1)
+  int64_t lp;           // row length of sk (launch_dct_literal)
+  double* sk;           // spectra, dct_sizes elements a tile
+  double* t1;           // after the x transform
+  double* t2;           // after the y transform
+  const double* tab[3];  // folded cosines of each axis (launch_dct_table)
+  Epilogue epi;         // output stage; nt > 1: plain tiles one after the other at epi.out
 };
 cudaError_t launch_dct_literal(const DctArgs& a, cudaStream_t s);
+// Elements of one tile's sk, t1 and t2.
+void dct_sizes(const int Np[3], const int K[3], int64_t* sk, int64_t* t1, int64_t* t2);
+// Folded cosine matrix of a transform of length N over K inputs: K rows of
+// round_up((N + 1) / 2, 2); ctab = cos(pi m / (2 N)), m < 4N.
+cudaError_t launch_dct_table(const double* ctab, int N, int K, double* tab, cudaStream_t s);
+
+// The blended field from all tiles of a sample held in memory (FP64).
+struct BlendGather {
+  const double* tiles;
+  double* out;
+  int Np[3], No[3], T[3];
+  int64_t L[3];
+  const double* sw[3];   // rank 0's sqrt weights per axis, rank r's sws r further
+  const uint8_t* fl[3];  // rank 0's flags per axis, rank r's fls r further
+  int64_t sws, fls;
+  int pou, marginal;
+  double ms, mu;
+};
+cudaError_t launch_blend_gather(const BlendGather& g, cudaStream_t s);
 
 // Post steps.
-cudaError_t launch_blend_tile(int dt, const void* tile, const int Np[3], const Epilogue& e,
-                              cudaStream_t s);
 cudaError_t launch_apply_pou(int dt, void* field, const int Np[3], const BlendAxis ax[3],
                              cudaStream_t s);
 cudaError_t launch_add_overlap(const double* in, double* out, const int Np[3],
