@@ -3262,14 +3262,31 @@ int scarl_rebuild_sk(scarl_ctx* ctx, const void* field, int dtype, const int L[3
   const size_t n = (size_t)L[0] * L[1] * L[2];
   const void* dev;
   RC(in_dev(ctx, ctx->stage_in, field, n * dtype, &dev));
+  // per axis: Tukey window, power pass, lag sums; one upload, one read back
   const double r = (double)0.1f;  // SRC_F/Stat_ScaRL/statistics_RF.f90:277
-  int off = 0;
+  const size_t nw = (size_t)L[0] + L[1] + L[2];
+  int N[3], nb[3], nmax = 0;
+  size_t pbytes = 0;
   for (int d = 0; d < 3; ++d) {
-    const int nl = L[d];
-    const int nkeep = nl / 2;
-    std::vector<double> w(nl);
-    for (int i = 0; i < nl; ++i) {  // statistics_RF.f90:325-351
-      const double ratio = (double)i / (double)(nl - 1);
+    N[d] = line_power_length(L[d]);
+    nb[d] = N[d] ? line_power_blocks(dtype, L, d, N[d]) : -1;
+    if (nb[d] < 1) return fail(ctx, SCARL_EDEVICE, "no launch configuration for the lag sums");
+    pbytes = std::max(pbytes, (size_t)nb[d] * N[d] * 8);
+    nmax = std::max(nmax, N[d]);
+  }
+  const void* tw[3];
+  for (int d = 0; d < 3; ++d) RC(twiddles(ctx, N[d], 8, &tw[d]));
+  RC(ensure(ctx, ctx->part, pbytes));
+  RC(ensure(ctx, ctx->t2, ((size_t)nmax + nw) * 8));
+  RC(ensure(ctx, ctx->tabs, nw * 8));
+  double* bins = (double*)ctx->t2.p;
+  double* S = bins + nmax;
+  void* hp;
+  RC(pinned(ctx, nw * 8, &hp));
+  double* w = (double*)hp;
+  for (int d = 0; d < 3; w += L[d], ++d) {
+    for (int i = 0; i < L[d]; ++i) {  // statistics_RF.f90:325-351
+      const double ratio = (double)i / (double)(L[d] - 1);
       w[i] = 1.0;
       if (tukey_literal) {
         if (ratio < r) w[i] = 1.0 / 2.0 * (1 + std::cos(2.0 * kPiRef / r * (ratio - r / 2.0)));
@@ -3279,28 +3296,24 @@ int scarl_rebuild_sk(scarl_ctx* ctx, const void* field, int dtype, const int L[3
         else if (ratio > 1.0 - r / 2.0) w[i] = 1.0 / 2.0 * (1 + std::cos(2.0 * M_PI / r * (ratio - 1.0 + r / 2.0)));
       }
     }
-    void* hp;
-    RC(pinned(ctx, (size_t)nl * 8, &hp));
-    std::memcpy(hp, w.data(), (size_t)nl * 8);
-    RC(ensure(ctx, ctx->tabs, (size_t)nl * 8));
-    RC(upload_pinned(ctx, ctx->tabs.p, (size_t)nl * 8));
-    const int np = lag_cov_parts(L, d);
-    RC(ensure(ctx, ctx->part, (size_t)np * std::max(nkeep, 1) * 8));
-    {
-      Prof p(ctx, "k_lag_cov");
-      CK(launch_lag_cov(dtype, dev, L, d, avg, stdDev, (const double*)ctx->tabs.p, nkeep,
-                        (double*)ctx->part.p, np, ctx->stream));
-    }
-    std::vector<double> h((size_t)np * nkeep);
-    CK(cudaMemcpyAsync(h.data(), ctx->part.p, h.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    const double nlines = (double)(n / (size_t)nl);
-    for (int m = 0; m < nkeep; ++m) {
-      double s = 0.0;
-      for (int b = 0; b < np; ++b) s += h[(size_t)b * nkeep + m];
-      SkTot[off + m] = s / ((double)nl * nlines);
-    }
-    off += nkeep;
+  }
+  RC(upload_pinned(ctx, ctx->tabs.p, nw * 8));
+  size_t o = 0;
+  for (int d = 0; d < 3; o += L[d], ++d) {
+    Prof p(ctx, "k_line_power", 3);
+    CK(launch_line_power(dtype, dev, L, d, N[d], avg, (const double*)ctx->tabs.p + o, tw[d], (double*)ctx->part.p, nb[d],
+                         bins, S + o, ctx->stream));
+  }
+  std::vector<double> h(nw);
+  CK(cudaMemcpyAsync(h.data(), S, nw * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  ctx->d2h += nw * 8;
+  const double* R = h.data();
+  for (int d = 0; d < 3; R += L[d], ++d) {
+    const int nl = L[d], nkeep = nl / 2;
+    // linear lag sums: at N = 2 n - 2 the last one came twice
+    auto lin = [&](int j) { return j >= nl ? 0.0 : (N[d] == 2 * nl - 2 && j == nl - 1) ? 0.5 * R[j] : R[j]; };
+    for (int m = 0; m < nkeep; ++m) *SkTot++ = (lin(m) + lin(nl - m)) / (stdDev * stdDev * (double)n);
   }
   return SCARL_OK;
 }

@@ -487,16 +487,6 @@ cudaError_t dispatch(int dt, int dir, int N, CovGeom g, const int* L, int want, 
                   : run_power_n<float, false>(N, g, L, want, blocks, s);
 }
 
-// P_k = sum over blocks of the partial power (one thread per bin).
-__global__ void k_cov_bins(const double* __restrict__ partial, int nblocks, int nbins,
-                           double* __restrict__ bins) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nbins) return;
-  double s = 0.0;
-  for (int b = 0; b < nblocks; ++b) s += partial[(int64_t)b * nbins + k];
-  bins[k] = s;
-}
-
 // S(h) = (1/M) [P_0 + (-1)^h P_N + 2 sum_{k=1}^{N-1} P_k cos(2 pi k h / M)],
 // one block per lag, FP64.
 __global__ void k_cov_lags(const double* __restrict__ bins, int N, const double2* __restrict__ tw64,
@@ -539,7 +529,8 @@ cudaError_t launch_axis_power(int dt, const void* f, const int L[3], int dir, in
 
 cudaError_t launch_cov_lags(const double* partial, int nblocks, int N, int maxlag,
                             const double* tw64, double* bins, double* S, cudaStream_t s) {
-  k_cov_bins<<<(N + 1 + 255) / 256, 256, 0, s>>>(partial, nblocks, N + 1, bins);
+  const cudaError_t e = launch_bins(partial, nblocks, N + 1, bins, s);
+  if (e != cudaSuccess) return e;
   k_cov_lags<<<maxlag + 1, 256, 0, s>>>(bins, N, reinterpret_cast<const double2*>(tw64), S);
   return cudaGetLastError();
 }

@@ -194,11 +194,16 @@ cudaError_t launch_sums(int dt, const void* f, int64_t xN, int nmc, double* part
                         cudaStream_t s);
 int sums_blocks(int64_t xN);
 
-// Directional circular autocovariance of the standardised, windowed field.
-cudaError_t launch_lag_cov(int dt, const void* f, const int L[3], int dir, double avg,
-                           double sd, const double* win, int nkeep, double* partial, int nparts,
-                           cudaStream_t s);
-int lag_cov_parts(const int L[3], int dir);
+// Directional autocovariance of the centred, windowed field (stats.cu): lines
+// of n points along axis dir in transforms of length N = line_power_length(n)
+// (0: none), partial holding nblocks x N doubles and bins N; S(j), j < n, gets
+// R(j) + R(N - j) of the linear lag sums R.  tw: FP64 e^{2 pi i m / N}.
+int line_power_length(int n);
+int line_power_blocks(int dt, const int L[3], int dir, int N);
+cudaError_t launch_line_power(int dt, const void* f, const int L[3], int dir, int N, double avg, const double* win,
+                              const void* tw, double* partial, int nblocks, double* bins, double* S, cudaStream_t s);
+// bins[k] = sum over rows of partial (nrows x nbins).
+cudaError_t launch_bins(const double* partial, int nrows, int nbins, double* bins, cudaStream_t s);
 
 // Streamed axis covariance (cov.cu): per-block FP64 power of the centred,
 // zero-padded lines along axis dir (complex length N, padded length 2N),
