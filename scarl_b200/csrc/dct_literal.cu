@@ -151,8 +151,8 @@ __global__ void __launch_bounds__(256, 2) k_dct_mm(const DctMM p) {
   auto slot_row = [](int row, int ld) { return ((row & 1) * kMmKB + (row >> 1)) * ld; };
   const unsigned da = sm0 + 8 * (slot_row(ra, Cfg::SA) + qa);
   const unsigned db = sm0 + 8 * (2 * kMmKB * Cfg::SA + slot_row(rb, Cfg::SB) + qb);
-  const double *pa, *pb;
-  int ka, kb_;
+  const double *pa = nullptr, *pb = nullptr;
+  int ka = 0, kb_ = 0;
   auto load = [&](int kb, int slot) {
     const int i0 = 2 * kMmKB * kb;
     const unsigned so = slot * (Cfg::STAGE * 8);

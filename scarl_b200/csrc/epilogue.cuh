@@ -1,5 +1,4 @@
-// epilogue.cuh -- per-point output stage shared by the C2R pass and the
-// tile-blend kernel: plain crop, or partition-of-unity blend into the global
+// epilogue.cuh -- per-point output stage of the C2R pass: plain crop, or partition-of-unity blend into the global
 // field (SRC_F/main_ScaRL.f90:1216-1301 weights, 984-1210 overlap sum,
 // write_output.f90:373-431 assembly) with the marginal transform
 // (SRC_F/main_ScaRL.f90:1355-1395) applied by the tile that finishes a point.
@@ -169,24 +168,6 @@ struct LineEpilogue {
       o[xs[i]] = w;
     }
   }
-  __device__ __forceinline__ void put(int x, T v) const {
-    if (mode == 0) {
-      out[base + x] = marg(v);
-      return;
-    }
-    const uint8_t f = fyz & fx[x];
-    if (!(f & 1)) return;
-    if (pou) v = v * (syz * sx[x]);
-    if (!(f & 2)) v = out[base + x] + v;
-    if (f & 4) v = marg(v);
-    out[base + x] = v;
-  }
 };
-
-template <typename T>
-__device__ __forceinline__ void epilogue_point(const Epilogue& e, int x, int y, int z, int Nx,
-                                               int Ny, T v) {
-  LineEpilogue<T>(e, y, z, Nx, Ny).put(x, v);
-}
 
 }  // namespace scarl

@@ -68,6 +68,27 @@ template <typename T> __device__ __forceinline__ T powT(T s, T e);
 template <> __device__ __forceinline__ float powT<float>(float s, float e) { return powf(s, e); }
 template <> __device__ __forceinline__ double powT<double>(double s, double e) { return pow(s, e); }
 
+// b^(-n/2) for b >= 1: a half-integer Matern order nu has n = nu + 3/2 whole,
+// and powers of 1 / sqrt(b) replace the general power (FP32: the hardware
+// approximation and one Newton step, relative error about 2^-23 before the
+// n - 1 products).
+__device__ __forceinline__ float rsqrt_acc(float b) {
+  const float y = rsqrtf(b);
+  return __fmaf_rn(0.5f * y, __fmaf_rn(-b * y, y, 1.0f), y);
+}
+__device__ __forceinline__ double rsqrt_acc(double b) { return rsqrt(b); }
+template <typename T> __device__ __forceinline__ T rsq_pow(T b, int n) {
+  const T y = rsqrt_acc(b);
+  T p = y;
+  for (int i = 1; i < n; ++i) p *= y;
+  return p;
+}
+// n of rsq_pow for the exponent expo = -n / 2, 0 where the general power runs.
+__device__ __forceinline__ int rsq_order(double expo) {
+  const double n = -2.0 * expo;
+  return n == floor(n) && n >= 2.0 && n <= 8.0 ? (int)n : 0;
+}
+
 // ---------------------------------------------------------------------------
 // Pass 1: synthesise + inverse DFT along z.
 // ---------------------------------------------------------------------------
@@ -93,18 +114,48 @@ __device__ __forceinline__ void gen_z_body(const GenArgs& a, int bx, int ky) {
       else { fx = ax[kx]; fy = T(1) + qx[kx] + qy[ky]; }
     }
   }
-  const uint64_t mrow = (uint64_t)kx + (uint64_t)a.Hx * (uint64_t)ky;
-  const uint64_t mz = (uint64_t)a.Hx * (uint64_t)a.P[1];
+  const int rsn = SPEC != SPEC_SHINO && a.amp == AMP_POW ? rsq_order(a.expo) : 0;
   auto amp = [&](int kz) -> T {
     if (a.amp == AMP_SEPARABLE) return fx * fy * az[kz];
     if (a.amp == AMP_RECIP) return fast_div(fx, fy + qz[kz]);
-    return fx * powT<T>(fy + qz[kz], (T)a.expo);
+    return fx * (rsn ? rsq_pow<T>(fy + qz[kz], rsn) : powT<T>(fy + qz[kz], (T)a.expo));
   };
   // First-stage inputs kz = j + r N/R1; r and r + R1/2 are kz and kz + N/2,
   // the two modes of one Philox draw.
+  constexpr int R1 = StagePlan<N, E>::radix(0), H = R1 / 2;
+  if constexpr (SPEC == SPEC_PHILOX) {
+    // The thread's draws in a loop, through its own slots of the line buffer
+    // (element kz at kz B + b): unrolled into the first stage they were some
+    // 1000 instructions with a power and two branches each, and the kernel
+    // waited on instruction fetches (2.2 of 10.8 stalled warps per issue).
+    // As a loop, with 32-bit counters and flushed hardware functions: 348 ->
+    // 284 us on a 512^3 grid (201 planes kept), FP64 122 -> 100 us on 256 x 224 x 256.
+    constexpr int TPL = N / E;
+    if (valid) {
+      const PhiloxLine draw(a.ks, a.stream);
+      const uint32_t c0 = (uint32_t)kx + (uint32_t)a.Hx * (uint32_t)ky, mz = (uint32_t)a.Hx * (uint32_t)a.P[1];
+#pragma unroll(sizeof(T) == 4 ? 2 : 1)
+      for (int d = 0; d < E / 2; ++d) {
+        const int kz = t + TPL * (d / H) + (d % H) * (N / R1);
+        const u32x4 o = draw(c0 + mz * (uint32_t)kz);
+        const C x0 = Normals<T>::from(o.x, o.y), x1 = Normals<T>::from(o.z, o.w);
+        const T A0 = amp(kz), A1 = amp(kz + N / 2);
+        sm[kz * B + b] = mk(A0 * x0.x, A0 * x0.y);
+        sm[(kz + N / 2) * B + b] = mk(A1 * x1.x, A1 * x1.y);
+      }
+    } else {
+#pragma unroll
+      for (int d = 0; d < E; ++d) sm[(t + TPL * (d / R1) + (d % R1) * (N / R1)) * B + b] = mk(T(0), T(0));
+    }
+  }
   auto load = [&](int j, C* v) {
-    constexpr int R1 = StagePlan<N, E>::radix(0);
-    constexpr int H = R1 / 2;
+    if constexpr (SPEC == SPEC_PHILOX) {
+#pragma unroll
+      for (int r = 0; r < R1; ++r) v[r] = sm[(j + r * (N / R1)) * B + b];
+      return;
+    }
+    const uint64_t mrow = (uint64_t)kx + (uint64_t)a.Hx * (uint64_t)ky;
+    const uint64_t mz = (uint64_t)a.Hx * (uint64_t)a.P[1];
 #pragma unroll
     for (int r = 0; r < H; ++r) {
       const int kz0 = j + r * (N / R1), kz1 = kz0 + N / 2;
@@ -116,17 +167,9 @@ __device__ __forceinline__ void gen_z_body(const GenArgs& a, int bx, int ky) {
       if constexpr (SPEC == SPEC_SHINO) {
         v[r] = shino_mode<T>(a, kx, ky, kz0);
         v[r + H] = shino_mode<T>(a, kx, ky, kz1);
-      } else {
-        C x0, x1;
-        if constexpr (SPEC == SPEC_INJECT) {
-          x0 = static_cast<const C*>(a.xi)[mrow + mz * (uint64_t)kz0];
-          x1 = static_cast<const C*>(a.xi)[mrow + mz * (uint64_t)kz1];
-        } else {
-          const uint64_t c = mrow + mz * (uint64_t)kz0;
-          const u32x4 o = philox4x32_10_ks({(uint32_t)c, (uint32_t)(c >> 32), a.stream, 0u}, a.ks);
-          x0 = Normals<T>::from(o.x, o.y);
-          x1 = Normals<T>::from(o.z, o.w);
-        }
+      } else if constexpr (SPEC == SPEC_INJECT) {
+        const C x0 = static_cast<const C*>(a.xi)[mrow + mz * (uint64_t)kz0];
+        const C x1 = static_cast<const C*>(a.xi)[mrow + mz * (uint64_t)kz1];
         const T A0 = amp(kz0), A1 = amp(kz1);
         v[r] = mk(A0 * x0.x, A0 * x0.y);
         v[r + H] = mk(A1 * x1.x, A1 * x1.y);

@@ -76,15 +76,15 @@ constexpr uint64_t kWaitNs = 1000000000ull;  // 1 s per tensor-core wait
 
 // The canonical Box-Muller pair of Normals<float> (u1 = (a + 1/2) 2^-32,
 // u2 = (b + 1/2) 2^-32, r (cos 2 pi u2, sin 2 pi u2), r = sqrt(-2 ln u1)) at
-// the split path's accuracy: r as t rsqrt(t) (0 at t = 0) and u2 from the top 23 bits of
-// b (phase error <= 2 pi 2^-24), both far below the 2^-17 of the BF16 split.
+// the split path's accuracy: the phase 2 pi (u2 - 1/2) from the top 23 bits of
+// b as the mantissa of m in [1, 2), by one fused multiply-add and without a
+// conversion (phase error under 2^-21, far below the 2^-17 of the BF16 split).
 __device__ __forceinline__ float2 split_normals(uint32_t a, uint32_t b) {
+  constexpr float k2Pi = 6.28318530717958647692f;
   const float u1 = __fmaf_rn((float)a, 0x1p-32f, 0x1p-33f);
-  const float u2 = __uint_as_float(0x3F800000u | (b >> 9)) - 1.5f + 0x1p-24f;  // u2 - 1/2
-  const float t = -2.0f * __logf(u1);            // 0 when u1 rounds to 1
-  const float r = t * rsqrtf(fmaxf(t, 0x1p-100f));
+  const float r = sqrt_ftz(-1.38629436111989061883f * lg2_ftz(u1));
   float s, c;
-  __sincosf(6.28318530717958647692f * u2, &s, &c);
+  sincos_ftz(__fmaf_rn(__uint_as_float(0x3F800000u | (b >> 9)), k2Pi, (-1.5f + 0x1p-24f) * k2Pi), &s, &c);
   return make_float2(-r * c, -r * s);
 }
 
@@ -93,7 +93,7 @@ __device__ __forceinline__ float2 split_normals(uint32_t a, uint32_t b) {
 // amplitude (e = -(nu + 3/2) / 2), far below the 2^-17 of the BF16 split.
 __device__ __forceinline__ float pow_split(float b, float e) {
   float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e * __log2f(b)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e * lg2_ftz(b)));
   return r;
 }
 
@@ -210,7 +210,7 @@ __device__ __forceinline__ void gen_z_tc_body(const GenArgs& a0, const GenArgs* 
     }
     const GenArgs& a = BATCH ? sa : a0;
     const int nlines = a.Hx * a.P[1];  // <= 1025 * 2048
-    const uint64_t mz = (uint64_t)a.Hx * (uint64_t)a.P[1];
+    const uint32_t mz = (uint32_t)a.Hx * (uint32_t)a.P[1];
     const float* ax = static_cast<const float*>(a.ax);
     const float* ay = static_cast<const float*>(a.ay);
     const float* qx = static_cast<const float*>(a.qx);
@@ -238,12 +238,12 @@ __device__ __forceinline__ void gen_z_tc_body(const GenArgs& a0, const GenArgs* 
       // draw d (modes k2 = d and d + N2/2) fills K columns 4d .. 4d + 3, so
       // two draws make one 16-byte chunk
       const uint32_t rowoff = (uint32_t)((R1 >> 3) * Cfg::SBO1 + (R1 & 7) * 16);
-      // the Philox round keys and stream in registers for the item's draws
+      // the Philox round keys in registers for the item's draws
       // (a batch's argument block lives in shared memory beside the operands)
       uint32_t kr[20];
 #pragma unroll
       for (int r = 0; r < 20; ++r) kr[r] = a.ks[r];
-      const uint32_t strm = a.stream;
+      const PhiloxLine draw(kr, a.stream);
       auto put = [&](const float* v, int chunk) {
         uint4 h, t;
         tc::split2(v[0], v[1], h.x, t.x);
@@ -261,8 +261,7 @@ __device__ __forceinline__ void gen_z_tc_body(const GenArgs& a0, const GenArgs* 
         for (int e = 0; e < 4; ++e) {
           const int kz0 = s_k1 + N1 * (d0 + e);
           if (valid) {
-            const uint64_t c = (uint64_t)l + mz * (uint64_t)kz0;
-            const u32x4 o = philox4x32_10_ks({(uint32_t)c, (uint32_t)(c >> 32), strm, 0u}, kr);
+            const u32x4 o = draw((uint32_t)l + mz * (uint32_t)kz0);
             const float2 x0 = split_normals(o.x, o.y);
             const float2 x1 = split_normals(o.z, o.w);
             const float A0 = amp(kz0), A1 = amp(kz0 + N / 2);

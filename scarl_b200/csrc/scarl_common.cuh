@@ -62,24 +62,49 @@ __device__ __forceinline__ u32x4 philox4x32_10(u32x4 c, uint32_t k0, uint32_t k1
   return c;
 }
 
-// The same with the round keys precomputed (ks[r] = k0 + r 0x9E3779B9,
-// ks[10 + r] = k1 + r 0xBB67AE85): kernels read them from their parameter
-// block instead of rebuilding the schedule per draw.
-__device__ __forceinline__ u32x4 philox4x32_10_ks(u32x4 c, const uint32_t* ks) {
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    // each 32 x 32 -> 64-bit product as one wide multiply (both halves)
-    const uint64_t p0 = (uint64_t)0xD2511F53u * c.x;
-    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c.z;
-    u32x4 n;
-    n.x = (uint32_t)(p1 >> 32) ^ c.y ^ ks[r];
-    n.y = (uint32_t)p1;
-    n.z = (uint32_t)(p0 >> 32) ^ c.w ^ ks[10 + r];
-    n.w = (uint32_t)p0;
-    c = n;
+// The same for counters {c, 0, stream, 0} with the round keys precomputed
+// (ks[r] = k0 + r 0x9E3779B9, ks[10 + r] = k1 + r 0xBB67AE85).  The mode index
+// c of a padded grid fits 32 bits (at most 1025 x 2048 x 1024 draws), so what
+// does not depend on it is formed once per thread: round 1 keeps one product,
+// round 2 one, 18 of 20 in all.  Each 32 x 32 -> 64-bit product is one wide
+// multiply (both halves); they are what a draw costs (20 measured 80 cycles a
+// warp and scheduler, a quarter of the FP32 rate).
+struct PhiloxLine {
+  uint32_t z1, x2, z2, z3;  // key and stream parts of the first rounds' words
+  uint32_t w2;
+  const uint32_t* ks;
+  __device__ __forceinline__ PhiloxLine(const uint32_t* ks_, uint32_t stream) : ks(ks_) {
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * stream;
+    const uint32_t x1 = (uint32_t)(p1 >> 32) ^ ks[0];
+    const uint64_t p0 = (uint64_t)0xD2511F53u * x1;
+    z1 = ks[10];
+    x2 = (uint32_t)p1 ^ ks[1];
+    z2 = (uint32_t)(p0 >> 32) ^ ks[11];
+    w2 = (uint32_t)p0;
+    z3 = w2 ^ ks[12];
   }
-  return c;
-}
+  __device__ __forceinline__ u32x4 operator()(uint32_t c) const {
+    const uint64_t a = (uint64_t)0xD2511F53u * c;                        // round 1
+    const uint64_t b = (uint64_t)0xCD9E8D57u * ((uint32_t)(a >> 32) ^ z1);  // round 2
+    u32x4 v;
+    v.x = (uint32_t)(b >> 32) ^ x2;
+    v.y = (uint32_t)b;
+    v.z = (uint32_t)a ^ z2;
+    v.w = w2;
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+      const uint64_t p0 = (uint64_t)0xD2511F53u * v.x;
+      const uint64_t p1 = (uint64_t)0xCD9E8D57u * v.z;
+      u32x4 n;
+      n.x = (uint32_t)(p1 >> 32) ^ v.y ^ ks[r];
+      n.y = (uint32_t)p1;
+      n.z = (uint32_t)(p0 >> 32) ^ (r == 2 ? z3 : v.w ^ ks[10 + r]);
+      n.w = (uint32_t)p0;
+      v = n;
+    }
+    return v;
+  }
+};
 
 // Uniform in (0,1) from two 32-bit words: 52 random bits plus a half offset,
 // exactly representable, never 0 or 1.
@@ -104,17 +129,36 @@ template <> struct Normals<double> {
     return make_double2(r * c, r * s);
   }
 };
+// Hardware approximations with subnormals flushed (lg2, square root, sine and
+// cosine of an argument in radians): without .ftz each carries a rescaling
+// that the arguments here never need.
+__device__ __forceinline__ float lg2_ftz(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sqrt_ftz(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void sincos_ftz(float x, float* s, float* c) {
+  asm("sin.approx.ftz.f32 %0, %1;" : "=f"(*s) : "f"(x));
+  asm("cos.approx.ftz.f32 %0, %1;" : "=f"(*c) : "f"(x));
+}
 template <> struct Normals<float> {
   // Single precision, hardware transcendentals: u1 is formed with one
-  // rounding (relative error 2^-24, so small u1 keep their digits); the
-  // phase is reduced to (-pi, pi) where __sincosf is accurate, and the
-  // half-turn folded back by the sign.
+  // rounding (relative error 2^-24, so small u1 keep their digits).  The phase
+  // 2 pi (u2 - 1/2) in (-pi, pi), where the hardware sine is accurate, comes
+  // from the signed word b - 2^31 by one fused multiply-add: relative error
+  // 2^-24 of the reduced phase, not of u2.  The half-turn is the sign.
   static __device__ __forceinline__ float2 from(uint32_t a, uint32_t b) {
     const float u1 = __fmaf_rn((float)a, 0x1p-32f, 0x1p-33f);
-    const float u2 = __fmaf_rn((float)b, 0x1p-32f, 0x1p-33f);
-    const float r = sqrtf(-2.0f * __logf(u1));
+    const float r = sqrt_ftz(-1.38629436111989061883f * lg2_ftz(u1));  // -2 ln 2 lg2 u1 >= 0
+    const float ph = __fmaf_rn((float)(int32_t)(b ^ 0x80000000u), 6.28318530717958647692f * 0x1p-32f,
+                               6.28318530717958647692f * 0x1p-33f);
     float s, c;
-    __sincosf(6.28318530717958647692f * (u2 - 0.5f), &s, &c);
+    sincos_ftz(ph, &s, &c);
     return make_float2(-r * c, -r * s);
   }
 };
