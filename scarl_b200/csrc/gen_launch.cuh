@@ -7,6 +7,7 @@
 #include <type_traits>
 
 #include "c2r_shfl.cuh"
+#include "c2r_two.cuh"
 #include "gen_kernels.cuh"
 
 namespace scarl {
@@ -160,8 +161,32 @@ inline cudaError_t run_c2r_shfl(const GenArgs& a, const BatchMap* bm, int* block
 // with 8, 16 and 32 lanes a line (FP32).
 template <typename T> constexpr int kShflVars = std::is_same<T, float>::value ? 3 : 0;
 
+// Pass 3 in two in-register stages (c2r_two.cuh): needs the status word; one
+// FP64 moment pair a block.
+template <typename T, int N>
+inline cudaError_t run_c2r_two(const GenArgs& a, const BatchMap* bm, int* blocks, cudaStream_t s) {
+  using Cfg = TwoCfg<T, N>;
+  if constexpr (!Cfg::valid()) {
+    return cudaErrorInvalidConfiguration;
+  } else {
+    const int64_t nlines = (int64_t)a.Nout[1] * a.Nout[2];
+    const int64_t per_block = (int64_t)Cfg::WPB * Cfg::G * two_chunk(nlines, Cfg::WPB * Cfg::G, N);
+    const unsigned nb = (unsigned)((nlines + per_block - 1) / per_block);
+    if (blocks) {
+      *blocks = (int)nb;
+      return cudaSuccess;
+    }
+    if (!a.status) return cudaErrorInvalidValue;
+    if (bm) return launch_k(k_c2r_x_two_batch<T, N>, dim3(bm->total), dim3(Cfg::THREADS), Cfg::SMEM, s, *bm);
+    return launch_k(k_c2r_x_two<T, N>, dim3(nb), dim3(Cfg::THREADS), Cfg::SMEM, s, a);
+  }
+}
+// The engine variant of a pass 3 that the two-stage kernel takes the place of
+// where it serves the length.
+template <typename T> constexpr int kTwoRow = std::is_same<T, float>::value ? 4 : 2;
+
 // Variant v of pass `pass` for line length N (pass 3: N = P0/2).  Lengths
-// below 128 (64 for pass 3) have only variant 0; SPEC_INJECT / SPEC_SHINO
+// below 128 (64 for pass 3) have only variant 0 of the engine; SPEC_INJECT / SPEC_SHINO
 // pass-1 kernels only variant 0.
 template <typename T, int N>
 inline cudaError_t run_pass_n(int pass, int v, const GenArgs& a, const BatchMap* bm, int* nb,
@@ -218,6 +243,8 @@ inline cudaError_t run_pass_n(int pass, int v, const GenArgs& a, const BatchMap*
       if (v == RV::n + 1) return run_c2r_shfl<T, N, 16>(a, bm, nb, s);
       return run_c2r_shfl<T, N, 32>(a, bm, nb, s);
     }
+    if constexpr (TwoCfg<T, N>::valid())
+      if (v == kTwoRow<T>) return run_c2r_two<T, N>(a, bm, nb, s);
     if (v == 0) return run_c2r_x_v<T, N, RV::v[0].E, RV::v[0].B>(a, bm, nb, s);
     switch (v) {
       SCARL_ROWV(1)

@@ -91,13 +91,21 @@ int gen_pass3_partials(int dt, int v, const GenArgs& a) {
   return gen_pass_blocks(dt, 3, v, a);
 }
 
-// The variant an untuned (precision, pass, length) runs: the FP32 pass 3 on
-// the register transform with 32 lanes a line (else 16) where it serves the
-// length and the status word exists; variant 0 otherwise.
+// The variant an untuned (precision, pass, length) runs.  Pass 3: the
+// two-stage kernel where it serves the half length and the status word exists.
+// The exceptions are FP32 lines of 64 and 128 (two engine stages, no staging
+// of the outputs: 53.5 against 59.7 and 51.6 against 61.3 us on 256 x 2048 x
+// 256-point grids); elsewhere the two-stage kernel is the fastest of all
+// (FP32 half lengths 224 / 256 / 384 / 512: 47 / 45 / 48 / 65 us against 58 /
+// 62 / 66 / 72 for the best other; FP64 112 / 224 / 256: 46 / 45 / 46 against
+// 80 / 117 / 72).
 int gen_default_variant(int dt, int pass, const GenArgs& a) {
-  if (dt == 4 && pass == 3 && a.status) {
-    for (int v : {RowVars<float>::n + 2, RowVars<float>::n + 1})
-      if (gen_pass_blocks(dt, pass, v, a) > 0) return v;
+  if (pass == 3 && a.status) {
+    const int N = a.P[0] / 2;
+    if (dt == 4 && N == 64) return 3;
+    if (dt == 4 && N == 128) return 0;
+    const int v = dt == 4 ? kTwoRow<float> : kTwoRow<double>;
+    if (gen_pass_blocks(dt, pass, v, a) > 0) return v;
   }
   return 0;
 }
