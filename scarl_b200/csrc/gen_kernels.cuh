@@ -90,6 +90,44 @@ __device__ __forceinline__ int rsq_order(double expo) {
 }
 
 // ---------------------------------------------------------------------------
+// The Philox spectrum of nd draws of line (kx, ky), kx < Hx: draw d's modes
+// kz = kzof(d) and kz + N/2 go to put(kz, x).
+//
+// The draws run in a loop (through shared memory in the callers): unrolled into
+// the first DFT stage they were some 1000 instructions with a power and two
+// branches each, and the kernel waited on instruction fetches (2.2 of 10.8
+// stalled warps per issue).  As a loop, with 32-bit counters and flushed hardware
+// functions: 348 -> 284 us on a 512^3 grid (201 planes kept), FP64 122 -> 100 us
+// on 256 x 224 x 256.
+// ---------------------------------------------------------------------------
+template <typename T, class Kz, class Put>
+__device__ __forceinline__ void synth_line(const GenArgs& a, int kx, int ky, Kz kzof, int nd, int N, Put put) {
+  using C = cplx_t<T>;
+  const T* az = static_cast<const T*>(a.az);
+  const T* qz = static_cast<const T*>(a.qz);
+  T fx = static_cast<const T*>(a.ax)[kx], fy;
+  if (a.amp == AMP_SEPARABLE) fy = static_cast<const T*>(a.ay)[ky];
+  else fy = T(1) + static_cast<const T*>(a.qx)[kx] + static_cast<const T*>(a.qy)[ky];
+  const int rsn = a.amp == AMP_POW ? rsq_order(a.expo) : 0;
+  auto amp = [&](int kz) -> T {
+    if (a.amp == AMP_SEPARABLE) return fx * fy * az[kz];
+    if (a.amp == AMP_RECIP) return fast_div(fx, fy + qz[kz]);
+    return fx * (rsn ? rsq_pow<T>(fy + qz[kz], rsn) : powT<T>(fy + qz[kz], (T)a.expo));
+  };
+  const PhiloxLine draw(a.ks, a.stream);
+  const uint32_t c0 = (uint32_t)kx + (uint32_t)a.Hx * (uint32_t)ky, mz = (uint32_t)a.Hx * (uint32_t)a.P[1];
+#pragma unroll(sizeof(T) == 4 ? 2 : 1)
+  for (int d = 0; d < nd; ++d) {
+    const int kz = kzof(d);
+    const u32x4 o = draw(c0 + mz * (uint32_t)kz);
+    const C x0 = Normals<T>::from(o.x, o.y), x1 = Normals<T>::from(o.z, o.w);
+    const T A0 = amp(kz), A1 = amp(kz + N / 2);
+    put(kz, mk(A0 * x0.x, A0 * x0.y));
+    put(kz + N / 2, mk(A1 * x1.x, A1 * x1.y));
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Pass 1: synthesise + inverse DFT along z.
 // ---------------------------------------------------------------------------
 template <typename T, int N, int E, int B, int SPEC>
@@ -101,48 +139,29 @@ __device__ __forceinline__ void gen_z_body(const GenArgs& a, int bx, int ky) {
   const int kx = bx * B + b;
   const bool valid = kx < a.Hx;
   C* work = static_cast<C*>(a.work);
-  const T* ax = static_cast<const T*>(a.ax);
-  const T* ay = static_cast<const T*>(a.ay);
-  const T* az = static_cast<const T*>(a.az);
-  const T* qx = static_cast<const T*>(a.qx);
-  const T* qy = static_cast<const T*>(a.qy);
-  const T* qz = static_cast<const T*>(a.qz);
   T fx = T(0), fy = T(0);
-  if constexpr (SPEC != SPEC_SHINO) {
+  if constexpr (SPEC == SPEC_INJECT) {
     if (valid) {
-      if (a.amp == AMP_SEPARABLE) { fx = ax[kx]; fy = ay[ky]; }
-      else { fx = ax[kx]; fy = T(1) + qx[kx] + qy[ky]; }
+      fx = static_cast<const T*>(a.ax)[kx];
+      if (a.amp == AMP_SEPARABLE) fy = static_cast<const T*>(a.ay)[ky];
+      else fy = T(1) + static_cast<const T*>(a.qx)[kx] + static_cast<const T*>(a.qy)[ky];
     }
   }
-  const int rsn = SPEC != SPEC_SHINO && a.amp == AMP_POW ? rsq_order(a.expo) : 0;
   auto amp = [&](int kz) -> T {
-    if (a.amp == AMP_SEPARABLE) return fx * fy * az[kz];
-    if (a.amp == AMP_RECIP) return fast_div(fx, fy + qz[kz]);
-    return fx * (rsn ? rsq_pow<T>(fy + qz[kz], rsn) : powT<T>(fy + qz[kz], (T)a.expo));
+    if (a.amp == AMP_SEPARABLE) return fx * fy * static_cast<const T*>(a.az)[kz];
+    const T d = fy + static_cast<const T*>(a.qz)[kz];
+    return a.amp == AMP_RECIP ? fast_div(fx, d) : fx * powT<T>(d, (T)a.expo);
   };
   // First-stage inputs kz = j + r N/R1; r and r + R1/2 are kz and kz + N/2,
   // the two modes of one Philox draw.
   constexpr int R1 = StagePlan<N, E>::radix(0), H = R1 / 2;
   if constexpr (SPEC == SPEC_PHILOX) {
-    // The thread's draws in a loop, through its own slots of the line buffer
-    // (element kz at kz B + b): unrolled into the first stage they were some
-    // 1000 instructions with a power and two branches each, and the kernel
-    // waited on instruction fetches (2.2 of 10.8 stalled warps per issue).
-    // As a loop, with 32-bit counters and flushed hardware functions: 348 ->
-    // 284 us on a 512^3 grid (201 planes kept), FP64 122 -> 100 us on 256 x 224 x 256.
+    // the thread's draws through its own slots of the line buffer (element kz
+    // at kz B + b)
     constexpr int TPL = N / E;
     if (valid) {
-      const PhiloxLine draw(a.ks, a.stream);
-      const uint32_t c0 = (uint32_t)kx + (uint32_t)a.Hx * (uint32_t)ky, mz = (uint32_t)a.Hx * (uint32_t)a.P[1];
-#pragma unroll(sizeof(T) == 4 ? 2 : 1)
-      for (int d = 0; d < E / 2; ++d) {
-        const int kz = t + TPL * (d / H) + (d % H) * (N / R1);
-        const u32x4 o = draw(c0 + mz * (uint32_t)kz);
-        const C x0 = Normals<T>::from(o.x, o.y), x1 = Normals<T>::from(o.z, o.w);
-        const T A0 = amp(kz), A1 = amp(kz + N / 2);
-        sm[kz * B + b] = mk(A0 * x0.x, A0 * x0.y);
-        sm[(kz + N / 2) * B + b] = mk(A1 * x1.x, A1 * x1.y);
-      }
+      synth_line<T>(a, kx, ky, [&](int d) { return t + TPL * (d / H) + (d % H) * (N / R1); }, E / 2, N,
+                    [&](int kz, C x) { sm[kz * B + b] = x; });
     } else {
 #pragma unroll
       for (int d = 0; d < E; ++d) sm[(t + TPL * (d / R1) + (d % R1) * (N / R1)) * B + b] = mk(T(0), T(0));

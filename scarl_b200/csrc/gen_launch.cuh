@@ -9,6 +9,7 @@
 #include "c2r_shfl.cuh"
 #include "c2r_two.cuh"
 #include "gen_kernels.cuh"
+#include "gen_two.cuh"
 
 namespace scarl {
 
@@ -181,8 +182,29 @@ inline cudaError_t run_c2r_two(const GenArgs& a, const BatchMap* bm, int* blocks
     return launch_k(k_c2r_x_two<T, N>, dim3(nb), dim3(Cfg::THREADS), Cfg::SMEM, s, a);
   }
 }
-// The engine variant of a pass 3 that the two-stage kernel takes the place of
-// where it serves the length.
+// Passes 1 and 2 in two in-register stages (gen_two.cuh; pass 1: the Philox
+// spectrum only).
+template <typename T, int N>
+inline cudaError_t run_col_two(int pass, const GenArgs& a, const BatchMap* bm, int* blocks, cudaStream_t s) {
+  using Cfg = ColCfg<T, N>;
+  if constexpr (!Cfg::valid()) {
+    return cudaErrorInvalidConfiguration;
+  } else {
+    const dim3 grid((a.Hx + Cfg::LB - 1) / Cfg::LB, pass == 1 ? a.P[1] : a.Nout[2], 1), block(Cfg::THREADS);
+    if (blocks) {
+      *blocks = (int)(grid.x * grid.y);
+      return cudaSuccess;
+    }
+    if (bm)
+      return pass == 1 ? launch_k(k_gen_z_two_batch<T, N>, dim3(bm->total), block, Cfg::SMEM, s, *bm)
+                       : launch_k(k_mid_y_two_batch<T, N>, dim3(bm->total), block, Cfg::SMEM, s, *bm);
+    return pass == 1 ? launch_k(k_gen_z_two<T, N>, grid, block, Cfg::SMEM, s, a)
+                     : launch_k(k_mid_y_two<T, N>, grid, block, Cfg::SMEM, s, a);
+  }
+}
+// The engine variants that the two-stage kernels take the place of where they
+// serve the length: passes 1 and 2, pass 3.
+template <typename T> constexpr int kTwoCol = std::is_same<T, float>::value ? 5 : 3;
 template <typename T> constexpr int kTwoRow = std::is_same<T, float>::value ? 4 : 2;
 
 // Variant v of pass `pass` for line length N (pass 3: N = P0/2).  Lengths
@@ -224,6 +246,8 @@ inline cudaError_t run_pass_n(int pass, int v, const GenArgs& a, const BatchMap*
     return cudaErrorInvalidConfiguration;
   }
   if (pass == 1 || pass == 2) {
+    if constexpr (ColCfg<T, N>::valid())
+      if (v == kTwoCol<T>) return run_col_two<T, N>(pass, a, bm, nb, s);
     if (v == 0) {
       if (pass == 1) return run_gen_z_v<T, N, CV::v[0].E, CV::v[0].B, SPEC_PHILOX>(a, bm, nb, s);
       return run_mid_y_v<T, N, CV::v[0].E, CV::v[0].B>(a, bm, nb, s);

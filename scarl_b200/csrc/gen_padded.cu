@@ -70,7 +70,8 @@ cudaError_t launch_gen_pass(int dt, int pass, const GenArgs& a_in, cudaStream_t 
   if (pass == 1 && a.split && dt == 4 && a.spec == SPEC_PHILOX && gen_z_tc_supported(a.P[2]))
     return launch_gen_z_tc(a, s);
   if (pass == 3 && c2r_x_tc_used(dt, a)) return launch_c2r_x_tc(a, s);
-  return run_pass_dt(dt, pass, a.var[pass - 1], a, nullptr, nullptr, s);
+  // injected and literal spectra run the first pass-1 variant only
+  return run_pass_dt(dt, pass, pass == 1 && a.spec != SPEC_PHILOX ? 0 : a.var[pass - 1], a, nullptr, nullptr, s);
 }
 
 cudaError_t launch_gen_pass_batch(int dt, int pass, int v, const GenArgs& rep, const BatchMap& m,
@@ -91,23 +92,40 @@ int gen_pass3_partials(int dt, int v, const GenArgs& a) {
   return gen_pass_blocks(dt, 3, v, a);
 }
 
-// The variant an untuned (precision, pass, length) runs.  Pass 3: the
-// two-stage kernel where it serves the half length and the status word exists.
-// The exceptions are FP32 lines of 64 and 128 (two engine stages, no staging
-// of the outputs: 53.5 against 59.7 and 51.6 against 61.3 us on 256 x 2048 x
-// 256-point grids); elsewhere the two-stage kernel is the fastest of all
-// (FP32 half lengths 224 / 256 / 384 / 512: 47 / 45 / 48 / 65 us against 58 /
-// 62 / 66 / 72 for the best other; FP64 112 / 224 / 256: 46 / 45 / 46 against
-// 80 / 117 / 72).
+// The variant an untuned (precision, pass, length) runs: the fastest of a sweep
+// of every variant over lengths 32 .. 2048 on grids of 12 - 24 M modes, crop mode.
+//
+// Passes 1 and 2: the two-stage kernels for lengths m 2^a (m = 3, 5, 7), whose
+// engine plans take four or five stages (FP32 pass 1 / pass 2, us: 224 69.8 /
+// 25.1 against 90.5 / 33.2, 384 66 / 24 against 70 / 30, 448 81 / 27 against 92 /
+// 35; FP64 224 98 / 27 against 138 / 33), and for short powers of two.  Longer
+// powers of two keep two or three engine stages, with 32 values a thread in the
+// FP32 pass 2 from 512 on (33.3 against 36.9, 1024 39.5 against 43.5) and eight in
+// the FP64 pass 1 (256 101 against 108, 1024 122 against 155).
+// Pass 3: the two-stage kernel where it serves the half length and the status
+// word exists (FP32 224 / 256 / 384 / 512: 47 / 45 / 48 / 65 against 58 / 62 / 66 /
+// 72 for the best other; FP64 112 / 224 / 256: 46 / 45 / 46 against 80 / 117 / 72),
+// except FP32 lines of 64 and 128 (two engine stages, no staging of the outputs:
+// 53.5 against 59.7 and 51.6 against 61.3).
 int gen_default_variant(int dt, int pass, const GenArgs& a) {
-  if (pass == 3 && a.status) {
+  const bool f32 = dt == 4;
+  if (pass == 3) {
     const int N = a.P[0] / 2;
-    if (dt == 4 && N == 64) return 3;
-    if (dt == 4 && N == 128) return 0;
-    const int v = dt == 4 ? kTwoRow<float> : kTwoRow<double>;
-    if (gen_pass_blocks(dt, pass, v, a) > 0) return v;
+    if (!a.status) return 0;
+    if (f32 && N == 64) return 3;
+    if (f32 && N == 128) return 0;
+    const int v = f32 ? kTwoRow<float> : kTwoRow<double>;
+    return gen_pass_blocks(dt, pass, v, a) > 0 ? v : 0;
   }
-  return 0;
+  const int N = a.P[pass == 1 ? 2 : 1], two = f32 ? kTwoCol<float> : kTwoCol<double>;
+  const bool mixed = (N & (N - 1)) != 0;
+  if ((mixed || N <= (pass == 1 ? (f32 ? 256 : 64) : (f32 ? 32 : 64))) && gen_pass_blocks(dt, pass, two, a) > 0)
+    return two;
+  if (f32) {
+    if (pass == 1) return N >= 1024 ? 1 : 0;
+    return mixed ? (N > 1024 ? 1 : 0) : N >= 1024 ? 3 : N >= 512 ? 4 : 0;
+  }
+  return pass == 1 && !mixed && N >= 128 ? 2 : 0;
 }
 
 int gen_variant_count(int dt, int pass) {

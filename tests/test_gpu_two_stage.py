@@ -1,4 +1,5 @@
-"""Pass 3 in two in-register stages: every half length it serves, FP32 and FP64,
+"""The passes in two in-register stages.  Passes 1 and 2: every length they
+serve, partial groups of kx.  Pass 3: every half length it serves, FP32 and FP64,
 lines shorter and longer than its epilogue's groups of 128 and 64 values, one
 and several groups of lines a warp, crop and blend, streamed moments.
 Tolerances: the field gates (FP64 1e-12, FP32 1e-5 against the oracle)."""
@@ -56,3 +57,39 @@ def test_blend_and_moments(ctx, oracle, dtype, tol, xmax, pad, margi):
     # FP64 sums of n values: n 2^-53 relative at most
     assert abs(sums[0] - f.sum()) < 1e-9 * np.abs(f).sum()
     assert abs(sums[1] - (f * f).sum()) < 1e-9 * (f * f).sum()
+
+
+COL = [32, 48, 64, 80, 96, 112, 128, 160, 192, 224, 256, 320, 384, 448, 512, 640, 768, 896, 1024]
+
+
+@pytest.mark.parametrize("pass_", [1, 2])
+@pytest.mark.parametrize("N", COL)
+@pytest.mark.parametrize("dtype,tol,var", [(S.F64, 1e-12, 3), (S.F32, 1e-5, 5)])
+def test_lengths_columns(ctx, oracle, N, pass_, dtype, tol, var):
+    if dtype == S.F64 and N > 256:
+        pytest.skip("FP64 in two stages up to 256")
+    ctx.tune_set(dtype, pass_, N, var)
+    try:
+        for px, n in ((16, N), (32, N // 2 + 1), (64, 3)):  # Hx = 9, 17, 33: one kx past the groups
+            P = (px, 8, N) if pass_ == 1 else (px, N, 8)
+            Np = (px - 3, 5, n) if pass_ == 1 else (px - 3, n, 5)
+            ref = oracle.gen_padded(Np, P, (1, 1, 1), (4, 3, 5), 3, 0.5, 1, seed=8, stream=2)
+            out = S.gen_padded(ctx, Np, (1, 1, 1), (4, 3, 5), 3, pad=P, seed=8, stream=2, dtype=dtype)
+            assert rel(out, ref) < tol
+    finally:
+        ctx.tune_set(dtype, pass_, N, -1)
+
+
+def test_injected_normals_under_a_tuned_pass_1(ctx, oracle):
+    """Injected normals run the one pass-1 variant they have, whatever the
+    context is tuned to."""
+    Np, P = (12, 9, 20), (16, 16, 224)
+    rng = np.random.default_rng(4)
+    xi = rng.standard_normal((P[2], P[1], P[0] // 2 + 1, 2))
+    ctx.tune_set(S.F64, 1, 224, 3)
+    try:
+        out = S.gen_padded(ctx, Np, (1, 1, 1), (4, 3, 5), 3, pad=P, xi=xi, dtype=S.F64)
+    finally:
+        ctx.tune_set(S.F64, 1, 224, -1)
+    ref = oracle.gen_padded(Np, P, (1, 1, 1), (4, 3, 5), 3, 0.5, 1, xi=xi)
+    assert rel(out, ref) < 1e-12
