@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(cov_threads<T, N, ROW>(), cov_minb<T, N, ROW>(
   constexpr int B = cov_B<T, N, ROW>();
   constexpr int TPL = N / E;
   constexpr int NT = B * TPL;
-  constexpr int QB = (N + NT) / NT;  // bins per thread (bins 0..N)
+  constexpr int QB = (N / 2 + NT) / NT;  // pairs of bins (k, N - k) per thread, k = 0..N/2
   // lanes along a line (line-fast shared layout) only in the direct form of
   // x lines; the staged form transforms x lines like the column layouts
   // (lanes across lines), reading them from a line-major input buffer
@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(cov_threads<T, N, ROW>(), cov_minb<T, N, ROW>(
     __syncthreads();
     tw = tws;
   }
-  double acc[QB];
+  double acc[QB][2];
 #pragma unroll
-  for (int q = 0; q < QB; ++q) acc[q] = 0.0;
+  for (int q = 0; q < QB; ++q) acc[q][0] = acc[q][1] = 0.0;
   const int64_t ngroups = (g.nlines + B - 1) / B;
   const T mu = (T)g.mu;
   // First-stage inputs of this thread for the lines of group grp, centred and
@@ -301,22 +301,31 @@ __global__ void __launch_bounds__(cov_threads<T, N, ROW>(), cov_minb<T, N, ROW>(
     };
     line_ifft<C, N, E, O, B, LS, true, 2>(sm, b, t, tw, load, store);
     __syncthreads();
+    // bins k and N - k of a line come from the same two transform values
+    // (both times |E + w O|^2, E and O the even and odd samples' transforms):
+    // each pair is read once
+    auto power = [](C zk, C zn, C w) -> T {
+      const C zc = cconj(zn);
+      const C e = mk((zk.x + zc.x) * T(0.5), (zk.y + zc.y) * T(0.5));
+      // (zk - zc) / (2i)
+      const C od = mk((zk.y - zc.y) * T(0.5), -(zk.x - zc.x) * T(0.5));
+      const C y = cadd(e, cmul(w, od));
+      return y.x * y.x + y.y * y.y;
+    };
 #pragma unroll
     for (int q = 0; q < QB; ++q) {
       const int k = (int)threadIdx.x + NT * q;
-      if (k > N) break;
-      const C w = tw[k];
-      T s = T(0);
+      if (k > N / 2) break;
+      const C w0 = tw[k], w1 = tw[N - k];
+      T s0 = T(0), s1 = T(0);
+#pragma unroll 4
       for (int bb = 0; bb < B; ++bb) {
-        const C zk = sm[bb * (N + 1) + (k == N ? 0 : k)];
-        const C zc = cconj(sm[bb * (N + 1) + (k == 0 || k == N ? 0 : N - k)]);
-        const C e = mk((zk.x + zc.x) * T(0.5), (zk.y + zc.y) * T(0.5));
-        // (zk - zc) / (2i)
-        const C od = mk((zk.y - zc.y) * T(0.5), -(zk.x - zc.x) * T(0.5));
-        const C y = cadd(e, cmul(w, od));
-        s += y.x * y.x + y.y * y.y;
+        const C za = sm[bb * (N + 1) + k], zb = sm[bb * (N + 1) + (k == 0 ? 0 : N - k)];
+        s0 += power(za, zb, w0);
+        s1 += power(zb, za, w1);
       }
-      acc[q] += (double)s;
+      acc[q][0] += (double)s0;
+      acc[q][1] += (double)s1;
     }
     __syncthreads();
   }
@@ -331,7 +340,10 @@ __global__ void __launch_bounds__(cov_threads<T, N, ROW>(), cov_minb<T, N, ROW>(
 #pragma unroll
   for (int q = 0; q < QB; ++q) {
     const int k = (int)threadIdx.x + NT * q;
-    if (k <= N) g.partial[(int64_t)blockIdx.x * (N + 1) + k] = acc[q];
+    if (k > N / 2) break;
+    double* p = g.partial + (int64_t)blockIdx.x * (N + 1);
+    p[N - k] = acc[q][1];
+    p[k] = acc[q][0];  // k = N / 2: both are the same bin
   }
 }
 
