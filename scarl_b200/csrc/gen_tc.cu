@@ -108,23 +108,35 @@ __device__ __forceinline__ uint32_t kmaj_off(int row, int k, int sbo) {
 // (re k < L, im k >= L) or, with DRAW_ORDER, in the stage-1 operand's draw
 // order: k = 4 d + part with part 0 / 1 = re / im of input d, 2 / 3 = re / im
 // of input d + L / 2 (the two modes of one Philox draw).
+// The L roots are formed first (scratch: L words of split cosine and sine), the
+// matrix from them: with a sine and cosine per element the 6656 elements of the
+// 8 x 40 configuration were 10 us at the start of every launch.
+template <int L> __device__ void fill_roots(uint2* root) {
+  for (int m = threadIdx.x; m < L; m += blockDim.x) {
+    double s, c;
+    sincospi(2.0 * (double)m / (double)L, &s, &c);
+    auto split = [](double v) -> uint32_t {  // head in the low half, tail in the high half
+      const __nv_bfloat16 h = __double2bfloat16(v);
+      const __nv_bfloat16 t = __double2bfloat16(v - (double)__bfloat162float(h));
+      return (uint32_t)__bfloat16_as_ushort(h) | ((uint32_t)__bfloat16_as_ushort(t) << 16);
+    };
+    root[m] = make_uint2(split(c), split(s));
+  }
+}
 template <int L, int SBO, bool DRAW_ORDER>
-__device__ void fill_dft_b(unsigned char* hi, unsigned char* lo) {
+__device__ void fill_dft_b(const uint2* root, unsigned char* hi, unsigned char* lo) {
   for (int idx = threadIdx.x; idx < 4 * L * L; idx += blockDim.x) {
     const int n = idx / (2 * L), k = idx % (2 * L);
     const int no = n % L;
     const int ki = DRAW_ORDER ? k / 4 + ((k & 2) ? L / 2 : 0) : k % L;
     const bool im_in = DRAW_ORDER ? (k & 1) != 0 : k >= L;
-    const int m = (no * ki) % L;
-    double s, c;
-    sincospi(2.0 * (double)m / (double)L, &s, &c);
     const bool im_out = n >= L;
-    const double v = (im_out == im_in) ? c : (im_out ? s : -s);
-    const __nv_bfloat16 h = __double2bfloat16(v);
-    const __nv_bfloat16 t = __double2bfloat16(v - (double)__bfloat162float(h));
+    const uint2 r = root[(no * ki) % L];
+    // cosine on the diagonal blocks, sine below, minus sine above (both signs)
+    const uint32_t v = im_out == im_in ? r.x : (im_out ? r.y : r.y ^ 0x80008000u);
     const uint32_t off = kmaj_off(n, k, SBO);
-    *reinterpret_cast<__nv_bfloat16*>(hi + off) = h;
-    *reinterpret_cast<__nv_bfloat16*>(lo + off) = t;
+    *reinterpret_cast<uint16_t*>(hi + off) = (uint16_t)v;
+    *reinterpret_cast<uint16_t*>(lo + off) = (uint16_t)(v >> 16);
   }
 }
 
@@ -152,8 +164,14 @@ __device__ __forceinline__ void gen_z_tc_body(const GenArgs& a0, const GenArgs* 
 
   if (tid == 0) tc::mbar_init(bar, 1);
   if (warp == 0) tc::tmem_alloc(tc::smem_u32(tslot), Cfg::TMEM_COLS);
-  fill_dft_b<N2, Cfg::SBO1, true>(sm + Cfg::OFF_B1H, sm + Cfg::OFF_B1L);
-  fill_dft_b<N1, Cfg::SBO2, false>(sm + Cfg::OFF_B2H, sm + Cfg::OFF_B2L);
+  {  // roots in the operand region, free until the first item
+    uint2* root = reinterpret_cast<uint2*>(sm);
+    fill_roots<N2>(root);
+    fill_roots<N1>(root + N2);
+    __syncthreads();
+    fill_dft_b<N2, Cfg::SBO1, true>(root, sm + Cfg::OFF_B1H, sm + Cfg::OFF_B1L);
+    fill_dft_b<N1, Cfg::SBO2, false>(root + N2, sm + Cfg::OFF_B2H, sm + Cfg::OFF_B2L);
+  }
   float* zt = reinterpret_cast<float*>(sm + Cfg::OFF_ZT);
   float2* tw2 = reinterpret_cast<float2*>(sm + Cfg::OFF_TW);
   auto load_zt = [&](const GenArgs& g) {
