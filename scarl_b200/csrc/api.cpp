@@ -36,6 +36,14 @@ struct Buf {
   size_t n = 0;
 };
 
+// A pinned host buffer and the event of its last upload.
+constexpr int kPinSlots = 8;
+struct PinSlot {
+  void* p = nullptr;
+  size_t n = 0;
+  cudaEvent_t ev = nullptr;
+};
+
 struct PaddedPlan {
   int dt = 4;
   int amp = AMP_SEPARABLE;
@@ -154,9 +162,8 @@ struct scarl_ctx {
   Buf status;  // device word raised by kernels whose bounded waits expired
   Buf mom;     // FP64 partial pairs of the streamed moments (pass 3) and their sum
   int wait_test = 0;  // test hook of the bounded tensor-core waits
-  void* pin = nullptr;
-  size_t pin_n = 0;
-  cudaEvent_t pin_ev = nullptr;
+  PinSlot pins[kPinSlots];  // pinned staging of small uploads, used in turn
+  int pin_cur = 0;
   // device -> pinned host copies of finished z slabs, overlapped with the
   // generation of the remaining tiles
   cudaStream_t copy_stream = nullptr;
@@ -258,25 +265,32 @@ bool is_pinned_host(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
-// Pinned host staging for small tables; waits for the previous upload.
+// Pinned host staging for small tables: the next of kPinSlots buffers, once the
+// upload that last used it is done.  (With one buffer each upload waited for
+// the previous one, which sits in the stream behind the previous call's kernels:
+// the host never ran ahead of the GPU.)
 int pinned(scarl_ctx* ctx, size_t bytes, void** out) {
-  if (ctx->pin_ev) CK(cudaEventSynchronize(ctx->pin_ev));
-  if (ctx->pin_n < bytes) {
-    if (ctx->pin) cudaFreeHost(ctx->pin);
-    ctx->pin = nullptr;
-    ctx->pin_n = 0;
-    CK(cudaMallocHost(&ctx->pin, bytes));
-    ctx->pin_n = bytes;
+  ctx->pin_cur = (ctx->pin_cur + 1) % kPinSlots;
+  PinSlot& b = ctx->pins[ctx->pin_cur];
+  if (b.ev) CK(cudaEventSynchronize(b.ev));
+  if (b.n < bytes) {
+    if (b.p) cudaFreeHost(b.p);
+    b.p = nullptr;
+    b.n = 0;
+    CK(cudaMallocHost(&b.p, bytes));
+    b.n = bytes;
   }
-  *out = ctx->pin;
+  *out = b.p;
   return SCARL_OK;
 }
 
+// Uploads the buffer that the last call of pinned returned.
 int upload_pinned(scarl_ctx* ctx, void* dst, size_t bytes) {
-  CK(cudaMemcpyAsync(dst, ctx->pin, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  PinSlot& b = ctx->pins[ctx->pin_cur];
+  CK(cudaMemcpyAsync(dst, b.p, bytes, cudaMemcpyHostToDevice, ctx->stream));
   ctx->h2d += bytes;
-  if (!ctx->pin_ev) CK(cudaEventCreateWithFlags(&ctx->pin_ev, cudaEventDisableTiming));
-  CK(cudaEventRecord(ctx->pin_ev, ctx->stream));
+  if (!b.ev) CK(cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming));
+  CK(cudaEventRecord(b.ev, ctx->stream));
   return SCARL_OK;
 }
 
@@ -1678,8 +1692,10 @@ int scarl_ctx_destroy(scarl_ctx* ctx) {
   ens_free(ctx);
   for (Buf* b : {&ctx->mlp_p, &ctx->mlp_m, &ctx->mlp_v, &ctx->mlp_g, &ctx->mlp_wb}) release(ctx, *b);
   for (cudaEvent_t e : ctx->pool) cudaEventDestroy(e);
-  if (ctx->pin_ev) cudaEventDestroy(ctx->pin_ev);
-  if (ctx->pin) cudaFreeHost(ctx->pin);
+  for (PinSlot& b : ctx->pins) {
+    if (b.ev) cudaEventDestroy(b.ev);
+    if (b.p) cudaFreeHost(b.p);
+  }
   for (cudaEvent_t e : ctx->slab_ev) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->ring_ev)
     if (e) cudaEventDestroy(e);
