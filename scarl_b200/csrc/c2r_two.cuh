@@ -51,8 +51,7 @@ template <typename T, int N> struct TwoCfg {
   static constexpr int OFF_TW = WPB * G * SLOT;          // e^{2 pi i k / 2N}, k < N
   static constexpr int OFF_T2 = OFF_TW + N * CB;         // e^{2 pi i m t / N} at m B + t
   static constexpr int OFF_SX = OFF_T2 + N * CB;         // s_x, x < 2N
-  static constexpr int OFF_FX = OFF_SX + 2 * N * (int)sizeof(T);
-  static constexpr int OFF_BAR = OFF_FX + (2 * N + 15) / 16 * 16;
+  static constexpr int OFF_BAR = OFF_SX + 2 * N * (int)sizeof(T);
   static constexpr int OFF_RED = OFF_BAR + WPB * 8;
   static constexpr int SMEM = OFF_RED + WPB * 16;
   static constexpr int R = A > B ? A : B;
@@ -74,24 +73,29 @@ __host__ __device__ inline int two_chunk(int64_t nlines, int per_block, int N) {
 __device__ __forceinline__ float two_exp(float x) { return __expf(x); }
 __device__ __forceinline__ double two_exp(double x) { return exp(x); }
 
-// K chunks of 32 x values of one line (C2R outputs at ob, destination o, lanes
-// along x, `left` values from this lane's first to the line's end): every read
-// of an earlier tile's partial sum before any write.
+// What the blend does along a line, as bounds on x (the flags along an axis are
+// an overlap, the inside, an overlap): x < add joins an earlier tile's partial
+// sum, x < fin is final (marginal), x < end is this tile's to store.  Three
+// compares a point; testing the flag bytes took 24 integer operations an output
+// where the crop takes 11.
+struct LineBounds {
+  int add, fin, end;
+};
+
+// K chunks of 32 x values of one line (C2R outputs at ob, destination o, the
+// lane's first value x): every read of an earlier tile's partial sum before any
+// write.
 template <typename T, int K, bool MOM, class Marg>
-__device__ __forceinline__ void two_blend(const T* ob, const T* sxs, const uint8_t* fxs, T* o, int left, int fyz, T syz,
-                                          Marg marg, double* s1, double* s2) {
+__device__ __forceinline__ void two_blend(const T* ob, const T* sxs, T* o, int x, const LineBounds& lb, T syz, Marg marg,
+                                          double* s1, double* s2) {
   T old[K];
-  int f[K];
+#pragma unroll
+  for (int u = 0; u < K; ++u) old[u] = x + 32 * u < lb.add ? o[32 * u] : T(0);
 #pragma unroll
   for (int u = 0; u < K; ++u) {
-    f[u] = 32 * u < left ? fyz & fxs[32 * u] : 0;
-    old[u] = (f[u] & 3) == 1 ? o[32 * u] : T(0);
-  }
-#pragma unroll
-  for (int u = 0; u < K; ++u) {
-    if (!(f[u] & 1)) continue;
+    if (x + 32 * u >= lb.end) continue;
     T w = old[u] + ob[32 * u] * (syz * sxs[32 * u]);
-    if (f[u] & 4) {
+    if (x + 32 * u < lb.fin) {
       w = marg(w);
       if constexpr (MOM) {
         *s1 += (double)w;
@@ -102,8 +106,8 @@ __device__ __forceinline__ void two_blend(const T* ob, const T* sxs, const uint8
   }
 }
 template <typename T, bool MOM>
-__device__ __forceinline__ void two_epilogue(const Epilogue& e, const T* ob, const T* sxs, const uint8_t* fxs, T* o,
-                                             int fyz, T syz, int lane, int Nx, double* s1, double* s2) {
+__device__ __forceinline__ void two_epilogue(const Epilogue& e, const T* ob, const T* sxs, T* o, const LineBounds& lb,
+                                             T syz, int lane, double* s1, double* s2) {
   const int marginal = e.marginal;
   const T ms = marginal ? (T)e.ms : T(1), mu = marginal ? (T)e.mmu : T(0);
   auto marg = [&](T v) -> T {
@@ -112,7 +116,7 @@ __device__ __forceinline__ void two_epilogue(const Epilogue& e, const T* ob, con
   };
   if (e.mode == 0) {
 #pragma unroll 4
-    for (int x = lane; x < Nx; x += 32) {
+    for (int x = lane; x < lb.end; x += 32) {
       const T w = marg(ob[x]);
       o[x] = w;
       if constexpr (MOM) {
@@ -125,9 +129,8 @@ __device__ __forceinline__ void two_epilogue(const Epilogue& e, const T* ob, con
   // groups of four chunks, the rest as one group of four or two
   int x = lane;
 #pragma unroll 1
-  for (; x - lane + 64 < Nx; x += 128)
-    two_blend<T, 4, MOM>(ob + x, sxs + x, fxs + x, o + x, Nx - x, fyz, syz, marg, s1, s2);
-  if (x - lane < Nx) two_blend<T, 2, MOM>(ob + x, sxs + x, fxs + x, o + x, Nx - x, fyz, syz, marg, s1, s2);
+  for (; x - lane + 64 < lb.end; x += 128) two_blend<T, 4, MOM>(ob + x, sxs + x, o + x, x, lb, syz, marg, s1, s2);
+  if (x - lane < lb.end) two_blend<T, 2, MOM>(ob + x, sxs + x, o + x, x, lb, syz, marg, s1, s2);
 }
 
 template <typename T, int N>
@@ -142,13 +145,14 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
   C* tws = reinterpret_cast<C*>(two_sm + Cfg::OFF_TW);
   C* tw2 = reinterpret_cast<C*>(two_sm + Cfg::OFF_T2);
   T* sxs = reinterpret_cast<T*>(two_sm + Cfg::OFF_SX);
-  uint8_t* fxs = two_sm + Cfg::OFF_FX;
   const uint32_t bar = tc::smem_u32(two_sm + Cfg::OFF_BAR + warp * 8);
   const int Nx = a.Nout[0], Ny = a.Nout[1];
   const int nlines = Ny * a.Nout[2];  // at most 2048^2
   const int chunk = two_chunk(nlines, Cfg::WPB * G, N);
   const int l00 = ((int)bx * chunk * Cfg::WPB + warp) * G;  // the warp's first line; its groups are WPB G apart
   const bool blend = a.epi.mode != 0;
+  __shared__ LineBounds xb;  // along x alone
+  if (threadIdx.x == 0) xb = LineBounds{0, Nx, Nx};
   auto fetch = [&](int l0) {  // lane 0: the group's line copies
     const int nv = min(G, nlines - l0);
     mbar_expect_tx(bar, (uint32_t)(nv * Cfg::LINE_BYTES));
@@ -171,14 +175,20 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
     }
     if (blend) {
       const T* sx = sw_of<T>(a.epi.ax[0]);
-      const uint8_t* fx = a.epi.ax[0].flags;
-      for (int i = (int)threadIdx.x; i < Nx; i += Cfg::THREADS) {
-        sxs[i] = a.epi.apply_pou ? __ldg(sx + i) : T(1);
-        fxs[i] = __ldg(fx + i);
-      }
+      for (int i = (int)threadIdx.x; i < Nx; i += Cfg::THREADS) sxs[i] = a.epi.apply_pou ? __ldg(sx + i) : T(1);
     }
   }
-  __syncthreads();  // tables and the warps' barrier initialisation
+  __syncthreads();  // tables, the warps' barrier initialisation, xb
+  if (blend) {
+    const uint8_t* fx = a.epi.ax[0].flags;
+    for (int i = (int)threadIdx.x; i < Nx; i += Cfg::THREADS) {
+      const int f = __ldg(fx + i), n = i + 1 < Nx ? (int)__ldg(fx + i + 1) : 7, p = i > 0 ? (int)__ldg(fx + i - 1) : 7;
+      if (!(f & 2) && ((n & 2) || i + 1 == Nx)) xb.add = i + 1;
+      if (!(f & 4) && (p & 4)) xb.fin = i;
+      if (!(f & 1) && (p & 1)) xb.end = i;
+    }
+    __syncthreads();
+  }
   double s1 = 0.0, s2 = 0.0;
   const bool mom = a.epi.mom != nullptr;
   uint32_t phase = 0;
@@ -276,9 +286,12 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
       T* o = static_cast<T*>(a.epi.out) + __shfl_sync(0xffffffffu, base, i);
       const int fi = __shfl_sync(0xffffffffu, fyz, i);
       const T si = __shfl_sync(0xffffffffu, syz, i);
+      if (!(fi & 1)) continue;
+      const int end = xb.end;
+      const LineBounds lb{(fi & 2) ? min(xb.add, end) : end, (fi & 4) ? min(xb.fin, end) : 0, end};
       const T* ob = reinterpret_cast<const T*>(wreg + i * Cfg::SLOT);
-      if (mom) two_epilogue<T, true>(a.epi, ob, sxs, fxs, o, fi, si, lane, Nx, &s1, &s2);
-      else two_epilogue<T, false>(a.epi, ob, sxs, fxs, o, fi, si, lane, Nx, &s1, &s2);
+      if (mom) two_epilogue<T, true>(a.epi, ob, sxs, o, lb, si, lane, &s1, &s2);
+      else two_epilogue<T, false>(a.epi, ob, sxs, o, lb, si, lane, &s1, &s2);
     }
     __syncwarp();
     if (lane == 0 && c + 1 < chunk && l0 + Cfg::WPB * G < nlines) {
