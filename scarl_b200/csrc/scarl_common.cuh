@@ -18,6 +18,9 @@ __device__ __forceinline__ double2 mk(double x, double y) { return make_double2(
 
 template <typename C> __device__ __forceinline__ C cadd(C a, C b) { return mk(a.x + b.x, a.y + b.y); }
 template <typename C> __device__ __forceinline__ C csub(C a, C b) { return mk(a.x - b.x, a.y - b.y); }
+// FP32: one packed operation for both parts (the same two roundings)
+template <> __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+template <> __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   return mk(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
