@@ -1293,6 +1293,10 @@ int upload_blend_tables(scarl_ctx* ctx, const scarl_layout& lay, int partitionTy
       ax.sw64 = (const double*)(dbase + (od + 2 * (size_t)Np) * 8);
       ax.sw32 = (const float*)(dbase + dbytes + of * 4);
       ax.flags = (const uint8_t*)(dbase + dbytes + fbytes + of);
+      const uint8_t* fl = hb + of;
+      for (ax.add = 0; ax.add < Np && !(fl[ax.add] & 2);) ++ax.add;
+      for (ax.fin = Np; ax.fin > 0 && !(fl[ax.fin - 1] & 4);) --ax.fin;
+      for (ax.end = Np; ax.end > 0 && !(fl[ax.end - 1] & 1);) --ax.end;
       od += 3 * (size_t)Np;
       of += (size_t)Np;
     }
@@ -2749,7 +2753,9 @@ int scarl_generate_sample(scarl_ctx* ctx, const scarl_sample* s, const scarl_gen
   RC(upload_blend_tables(ctx, lay, 1, &axes));
   Epilogue epi;
   std::memset(&epi, 0, sizeof epi);
-  epi.mode = 1;
+  // a single tile is the field: the crop writes the same values (every weight
+  // is 1, every point first and last) without the blend's tables
+  epi.mode = lay.nb_tiles > 1 ? 1 : 0;
   epi.out = dev;
   for (int d = 0; d < 3; ++d) epi.L[d] = lay.L[d];
   epi.marginal = o.normalize_field ? 0 : s->margiFirst;

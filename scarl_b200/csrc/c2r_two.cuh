@@ -151,22 +151,27 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
   const int chunk = two_chunk(nlines, Cfg::WPB * G, N);
   const int l00 = ((int)bx * chunk * Cfg::WPB + warp) * G;  // the warp's first line; its groups are WPB G apart
   const bool blend = a.epi.mode != 0;
-  __shared__ LineBounds xb;  // along x alone
-  if (threadIdx.x == 0) xb = LineBounds{0, Nx, Nx};
-  auto fetch = [&](int l0) {  // lane 0: the group's line copies
+  // the group's lines: bulk copies issued by lane 0, or, for a caller without a
+  // status word to report an expired wait in, 16-byte cp.async by every lane
+  const bool bulk = a.status != nullptr;
+  auto fetch = [&](int l0) {
     const int nv = min(G, nlines - l0);
-    mbar_expect_tx(bar, (uint32_t)(nv * Cfg::LINE_BYTES));
     const C* work = static_cast<const C*>(a.work);
+    if (bulk && lane == 0) mbar_expect_tx(bar, (uint32_t)(nv * Cfg::LINE_BYTES));
     for (int i = 0; i < nv; ++i) {
       const int l = l0 + i, z = l / Ny, y = l - z * Ny;
-      bulk_g2s(tc::smem_u32(wreg + i * Cfg::SLOT), work + ((size_t)z * a.P[1] + (size_t)y) * a.Hpad, Cfg::LINE_BYTES,
-               bar);
+      const C* src = work + ((size_t)z * a.P[1] + (size_t)y) * a.Hpad;
+      unsigned char* dst = wreg + i * Cfg::SLOT;
+      if (!bulk) {
+        for (int c = lane; c < Cfg::LINE_BYTES / 16; c += 32)
+          cp_async16(dst + 16 * c, reinterpret_cast<const char*>(src) + 16 * c);
+      } else if (lane == 0) {
+        bulk_g2s(tc::smem_u32(dst), src, Cfg::LINE_BYTES, bar);
+      }
     }
   };
-  if (lane == 0) {
-    tc::mbar_init(bar, 1);
-    if (l00 < nlines) fetch(l00);
-  }
+  if (lane == 0) tc::mbar_init(bar, 1);
+  if (l00 < nlines) fetch(l00);
   {
     const C* twx = static_cast<const C*>(a.tw_x);
     for (int i = (int)threadIdx.x; i < N; i += Cfg::THREADS) {
@@ -178,17 +183,7 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
       for (int i = (int)threadIdx.x; i < Nx; i += Cfg::THREADS) sxs[i] = a.epi.apply_pou ? __ldg(sx + i) : T(1);
     }
   }
-  __syncthreads();  // tables, the warps' barrier initialisation, xb
-  if (blend) {
-    const uint8_t* fx = a.epi.ax[0].flags;
-    for (int i = (int)threadIdx.x; i < Nx; i += Cfg::THREADS) {
-      const int f = __ldg(fx + i), n = i + 1 < Nx ? (int)__ldg(fx + i + 1) : 7, p = i > 0 ? (int)__ldg(fx + i - 1) : 7;
-      if (!(f & 2) && ((n & 2) || i + 1 == Nx)) xb.add = i + 1;
-      if (!(f & 4) && (p & 4)) xb.fin = i;
-      if (!(f & 1) && (p & 1)) xb.end = i;
-    }
-    __syncthreads();
-  }
+  __syncthreads();  // tables and the warps' barrier initialisation
   double s1 = 0.0, s2 = 0.0;
   const bool mom = a.epi.mom != nullptr;
   uint32_t phase = 0;
@@ -196,7 +191,10 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
   for (int c = 0; c < chunk; ++c) {
     const int l0 = l00 + c * Cfg::WPB * G;
     if (l0 >= nlines) break;
-    if (!tc::mbar_wait(bar, phase, kBulkWaitNs)) {
+    if (!bulk) {
+      cp_async_wait_all();
+      __syncwarp();
+    } else if (!tc::mbar_wait(bar, phase, kBulkWaitNs)) {
       // a copy did not land in time: report, give it one more bounded wait
       // (the copies write this block's shared memory), leave the rest
       if (lane == 0) {
@@ -270,32 +268,38 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
     __syncwarp();
     // ---- epilogue: one line at a time, lanes along x; lane i < G holds what
     //      line i needs ----
-    unsigned long long base = 0;
-    int fyz = 0;
-    T syz = T(0);
+    long long base = 0;
+    int yz = 0;  // bit 0: contributes, bit 1: not the first, bit 2: the last
+    T syz = T(1);
     if (lane < G && l0 + lane < nlines) {
       const int l = l0 + lane, z = l / Ny, y = l - z * Ny;
-      const LineEpilogue<T> ep(a.epi, y, z, Nx, Ny);
-      base = ep.base;
-      fyz = ep.fyz;
-      syz = ep.syz;
+      const Epilogue& e = a.epi;
+      if (!blend) {
+        base = (long long)Nx * l;
+        yz = 5;
+      } else {
+        base = e.off[0] + e.L[0] * ((e.off[1] + y) + e.L[1] * (e.off[2] + z));
+        yz = (y < e.ax[1].end && z < e.ax[2].end ? 1 : 0) | (y < e.ax[1].add || z < e.ax[2].add ? 2 : 0) |
+             (y < e.ax[1].fin && z < e.ax[2].fin ? 4 : 0);
+        if (e.apply_pou) syz = sw_of<T>(e.ax[1])[y] * sw_of<T>(e.ax[2])[z];
+      }
     }
+    const LineBounds xb = blend ? LineBounds{a.epi.ax[0].add, a.epi.ax[0].fin, a.epi.ax[0].end} : LineBounds{0, Nx, Nx};
 #pragma unroll 1
     for (int i = 0; i < G; ++i) {
       if (l0 + i >= nlines) break;
       T* o = static_cast<T*>(a.epi.out) + __shfl_sync(0xffffffffu, base, i);
-      const int fi = __shfl_sync(0xffffffffu, fyz, i);
+      const int fi = __shfl_sync(0xffffffffu, yz, i);
       const T si = __shfl_sync(0xffffffffu, syz, i);
       if (!(fi & 1)) continue;
-      const int end = xb.end;
-      const LineBounds lb{(fi & 2) ? min(xb.add, end) : end, (fi & 4) ? min(xb.fin, end) : 0, end};
+      const LineBounds lb{(fi & 2) ? xb.end : min(xb.add, xb.end), (fi & 4) ? min(xb.fin, xb.end) : 0, xb.end};
       const T* ob = reinterpret_cast<const T*>(wreg + i * Cfg::SLOT);
       if (mom) two_epilogue<T, true>(a.epi, ob, sxs, o, lb, si, lane, &s1, &s2);
       else two_epilogue<T, false>(a.epi, ob, sxs, o, lb, si, lane, &s1, &s2);
     }
     __syncwarp();
-    if (lane == 0 && c + 1 < chunk && l0 + Cfg::WPB * G < nlines) {
-      tc::fence_smem_to_async();  // the warp's reads and writes before the copies'
+    if (c + 1 < chunk && l0 + Cfg::WPB * G < nlines) {
+      if (lane == 0) tc::fence_smem_to_async();  // the warp's reads and writes before the copies'
       fetch(l0 + Cfg::WPB * G);
     }
   }

@@ -9,16 +9,6 @@
 
 namespace scarl {
 
-// ---------------------------------------------------------------------------
-// Epilogue of one output point of a tile.
-// ---------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ T marginal_apply(const Epilogue& e, T v) {
-  if (e.marginal == 1) return v * (T)e.ms + (T)e.mmu;
-  if (e.marginal == 2) return exp(v * (T)e.ms + (T)e.mmu);
-  return v;
-}
-
 template <typename T> __device__ __forceinline__ const T* sw_of(const BlendAxis& a);
 template <> __device__ __forceinline__ const float* sw_of<float>(const BlendAxis& a) { return a.sw32; }
 template <> __device__ __forceinline__ const double* sw_of<double>(const BlendAxis& a) { return a.sw64; }

@@ -162,8 +162,7 @@ inline cudaError_t run_c2r_shfl(const GenArgs& a, const BatchMap* bm, int* block
 // with 8, 16 and 32 lanes a line (FP32).
 template <typename T> constexpr int kShflVars = std::is_same<T, float>::value ? 3 : 0;
 
-// Pass 3 in two in-register stages (c2r_two.cuh): needs the status word; one
-// FP64 moment pair a block.
+// Pass 3 in two in-register stages (c2r_two.cuh); one FP64 moment pair a block.
 template <typename T, int N>
 inline cudaError_t run_c2r_two(const GenArgs& a, const BatchMap* bm, int* blocks, cudaStream_t s) {
   using Cfg = TwoCfg<T, N>;
@@ -177,7 +176,6 @@ inline cudaError_t run_c2r_two(const GenArgs& a, const BatchMap* bm, int* blocks
       *blocks = (int)nb;
       return cudaSuccess;
     }
-    if (!a.status) return cudaErrorInvalidValue;
     if (bm) return launch_k(k_c2r_x_two_batch<T, N>, dim3(bm->total), dim3(Cfg::THREADS), Cfg::SMEM, s, *bm);
     return launch_k(k_c2r_x_two<T, N>, dim3(nb), dim3(Cfg::THREADS), Cfg::SMEM, s, a);
   }

@@ -102,16 +102,15 @@ int gen_pass3_partials(int dt, int v, const GenArgs& a) {
 // powers of two keep two or three engine stages, with 32 values a thread in the
 // FP32 pass 2 from 512 on (33.3 against 36.9, 1024 39.5 against 43.5) and eight in
 // the FP64 pass 1 (256 101 against 108, 1024 122 against 155).
-// Pass 3: the two-stage kernel where it serves the half length and the status
-// word exists (FP32 224 / 256 / 384 / 512: 47 / 45 / 48 / 65 against 58 / 62 / 66 /
-// 72 for the best other; FP64 112 / 224 / 256: 46 / 45 / 46 against 80 / 117 / 72),
-// except FP32 lines of 64 and 128 (two engine stages, no staging of the outputs:
-// 53.5 against 59.7 and 51.6 against 61.3).
+// Pass 3: the two-stage kernel where it serves the half length (FP32 224 / 256 /
+// 384 / 512: 47 / 45 / 48 / 65 against 58 / 62 / 66 / 72 for the best other; FP64
+// 112 / 224 / 256: 46 / 45 / 46 against 80 / 117 / 72), except FP32 lines of 64 and
+// 128 (two engine stages, no staging of the outputs: 53.5 against 59.7 and 51.6
+// against 61.3).
 int gen_default_variant(int dt, int pass, const GenArgs& a) {
   const bool f32 = dt == 4;
   if (pass == 3) {
     const int N = a.P[0] / 2;
-    if (!a.status) return 0;
     if (f32 && N == 64) return 3;
     if (f32 && N == 128) return 0;
     const int v = f32 ? kTwoRow<float> : kTwoRow<double>;

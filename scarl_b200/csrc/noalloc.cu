@@ -257,6 +257,8 @@ extern "C" int scarl_gen_padded_noalloc(void* out, int dtype, const int Np[3], c
   ga.stream = stream;
   ga.epi.mode = 0;
   ga.epi.out = out;
+  // the variants of an untuned context: the kernels that scarl_gen_padded runs
+  for (int pass = 1; pass <= 3; ++pass) ga.var[pass - 1] = gen_default_variant(dt, pass, ga);
   for (int pass = 1; pass <= 3; ++pass)
     if (launch_gen_pass(dt, pass, ga, s) != cudaSuccess)
       return say(msg, msg_len, SCARL_EDEVICE, "generator launch failed");

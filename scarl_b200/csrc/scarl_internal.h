@@ -18,6 +18,10 @@ struct BlendAxis {
   const uint8_t* flags;
   const double* sw64;  // sqrt(lo * hi): the axis' factor of sqrt(weight)
   const float* sw32;
+  // the flags as bounds (an overlap, the inside, an overlap): coordinates below
+  // add are not the first contributor's, below fin the last contributor's,
+  // below end contributed
+  int add, fin, end;
 };
 
 struct Epilogue {
