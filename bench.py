@@ -676,7 +676,7 @@ def main():
     ms_dct = timed_fn(step_dct, 3)
     dct_line = {"value": round(world * Np_t[0] * Np_t[1] * Np_t[2] / (ms_dct * 1e-3) / 1e6, 2),
                 "ms_per_tile": round(ms_dct, 3), "tile_points": Np_t,
-                "precision": "f64 (direct DCT-III sums on the CUDA cores)"}
+                "precision": "f64 (folded DCT-III products on the FP64 tensor cores)"}
     del dct_out
 
     # ---- per-kernel device times (separate, profiled steps)
