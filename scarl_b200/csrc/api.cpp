@@ -145,9 +145,11 @@ constexpr int kRingSlots = 4;
 constexpr size_t kRingChunk = (size_t)32 << 20;
 constexpr size_t kRingMin = (size_t)8 << 20;
 // literal DCT tiles generated and held together up to this many bytes: few
-// launches over all of them, the tiles staying in L2 for the gather (8 tiles of
-// 23^3: 45 us a sample against 250 us tile by tile); larger samples fill the
-// GPU with one tile and save the tiles' round trip through memory
+// launches over all of them, the tiles and the y step's output staying in the
+// 126 MB L2 for the gather.  8 tiles of 23^3, 66^3, 96^3 (0.8, 18, 57 MB): 58, 92,
+// 181 us a sample against 203, 271, 319 tile by tile; past the L2 the gain fades
+// (83 MB 84 against 115) and ends (252 MB 254 against 244, 941 MB 869 against 583),
+// where one tile fills the GPU and saves the tiles' round trip through memory
 constexpr size_t kDctBatch = (size_t)64 << 20;
 
 }  // namespace
@@ -2794,11 +2796,21 @@ int scarl_generate_sample(scarl_ctx* ctx, const scarl_sample* s, const scarl_gen
     for (int d = 0; d < 3; ++d)
       if (lay.Np[d] < 2) return fail(ctx, SCARL_EINVAL, "Np must be >= 2");
   }
-  // literal tiles that fit kDctBatch bytes together: one launch per step over
-  // all of them, then one gather of the blended field; larger ones one after
-  // the other, each blended by its z transform's output stage
-  const bool dct_batch = gen == SCARL_GEN_DCT && lay.nb_tiles > 1 && ntile * 8 * lay.nb_tiles <= kDctBatch &&
-                         ensure(ctx, ctx->tile, ntile * 8 * lay.nb_tiles) == SCARL_OK;
+  // literal tiles that fit kDctBatch bytes together, and the budget with their
+  // work buffers: one launch per step over all of them, then one gather of the
+  // blended field; larger ones one after the other, each blended by its z
+  // transform's output stage
+  bool dct_batch = gen == SCARL_GEN_DCT && lay.nb_tiles > 1 && ntile * 8 * lay.nb_tiles <= kDctBatch;
+  if (dct_batch) {
+    const int K[3] = {lay.Np[0] / 2, lay.Np[1] / 2, lay.Np[2] / 2};
+    int64_t nsk, n1, n2;
+    dct_sizes(lay.Np, K, &nsk, &n1, &n2);
+    const Buf* bufs[4] = {&ctx->tile, &ctx->sk, &ctx->t1, &ctx->t2};
+    const size_t want[4] = {ntile * 8, (size_t)nsk * 8, (size_t)n1 * 8, (size_t)n2 * 8};
+    size_t more = (size_t)1 << 20;  // the axes' tables
+    for (int i = 0; i < 4; ++i) more += want[i] * lay.nb_tiles > bufs[i]->n ? want[i] * lay.nb_tiles - bufs[i]->n : 0;
+    dct_batch = ctx->used + more <= ctx->budget && ensure(ctx, ctx->tile, ntile * 8 * lay.nb_tiles) == SCARL_OK;
+  }
   const void* phi_all = nullptr;
   if (gen == SCARL_GEN_DCT && o.phiK)
     RC(in_dev(ctx, ctx->stage_in, o.phiK, nk * lay.nb_tiles * 8, &phi_all));

@@ -61,3 +61,16 @@ def test_dct_lognormal_tile_after_tile(ctx, oracle):
     # cos of phases near a quarter turn: the two math libraries' cosines agree
     # to an ulp of 1, 2e-16 of values of 3e-5: 1e-11 relative
     assert rel(out - 1.0, ref - 1.0) < 1e-9
+
+
+def test_dct_small_budget(oracle):
+    """A context whose budget holds one tile's buffers but not all tiles'
+    together generates tile after tile."""
+    args = ((0, 0, 0), (90, 90, 90), (4, 4, 4), (1, 1, 1), (5, 5, 5))
+    ref, _ = oracle.generate_sample(1, *args, 1, 0.5, 1, 0.5, 2.0, 3, 8, (2, 2, 2))
+    s = S.make_sample(*args, 1, 1, 0.5, 2.0, 3)
+    # field 91^3: 6 MB staged; a 48^3 tile's spectrum and steps under 2 MB, 8
+    # tiles' buffers together over 12 MB
+    with S.Context(0, budget_bytes=12 << 20) as c:
+        out, _ = S.generate_sample(c, s, generator=S.GEN_DCT, dtype=S.F64, nb_procs=8, topo=(2, 2, 2))
+    assert rel(out, ref) < TOL64
