@@ -74,7 +74,8 @@ class Context:
         _check(lib().scarl_sync(self.handle), self)
 
     def tc_wait_test(self, enable=True):
-        """Test hook: the tensor-core pass's waits run out (SCARL_ETIMEOUT)."""
+        """Test hook: the tensor-core pass's waits and pass 3's line copies run out
+        (SCARL_ETIMEOUT)."""
         _check(lib().scarl_tc_wait_test(self.handle, int(bool(enable))), self)
 
     def profile(self, enable=True):

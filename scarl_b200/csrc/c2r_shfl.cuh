@@ -72,6 +72,16 @@ template <int N, int L> struct ShflCfg {
 
 constexpr uint64_t kBulkWaitNs = 1000000000ull;  // 1 s per line-copy wait
 
+// The warp's wait for its copies, with one outcome for all lanes: each lane
+// polls the barrier and the clock by itself, so a copy that lands at the limit
+// may count as landed for some and as late for others, and what follows (shuffles,
+// stores through shuffled bases) needs every lane.  test: the odd lanes count
+// every copy as late.
+__device__ __forceinline__ bool warp_bulk_wait(uint32_t mbar, uint32_t parity, int lane, int test) {
+  const bool ok = tc::mbar_wait(mbar, parity, kBulkWaitNs);
+  return __all_sync(0xffffffffu, ok && !(test && (lane & 1)));
+}
+
 // Epilogue of the KC x values x0 + lane + 32 j (j < KC) of one line whose
 // C2R outputs sit at ob (x < Nx <= 2N read).
 template <int KC, bool MOM>
@@ -140,7 +150,7 @@ __device__ __forceinline__ void c2r_shfl_body(const GenArgs& a, int64_t bx) {
   double s1 = 0.0, s2 = 0.0;
   const bool mom = a.epi.mom != nullptr;
   bool work_here = l0 < nlines;
-  if (work_here && !tc::mbar_wait(bar, 0, kBulkWaitNs)) {
+  if (work_here && !warp_bulk_wait(bar, 0, lane, a.wait_test)) {
     // a copy did not land in time: report, give it one more bounded wait
     // (the copies write this block's shared memory), skip the group
     if (lane == 0) {

@@ -194,7 +194,7 @@ __device__ __forceinline__ void c2r_two_body(const GenArgs& a, int64_t bx) {
     if (!bulk) {
       cp_async_wait_all();
       __syncwarp();
-    } else if (!tc::mbar_wait(bar, phase, kBulkWaitNs)) {
+    } else if (!warp_bulk_wait(bar, phase, lane, a.wait_test)) {
       // a copy did not land in time: report, give it one more bounded wait
       // (the copies write this block's shared memory), leave the rest
       if (lane == 0) {

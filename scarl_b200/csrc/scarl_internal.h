@@ -81,7 +81,8 @@ struct GenArgs {
   int var[3];            // launch variant of each pass (autotuned, 0 = default)
   int split;             // FP32, split BF16 on the tensor cores: bit 0 pass 1's z DFT, bit 1 pass 3's x DFT
   int* status;           // device word, bit 0 set when a bounded tensor-core wait expired
-  int wait_test;         // test hook: the tensor-core pass issues no MMA and waits 20 ms
+  int wait_test;         // test hook: the tensor-core pass issues no MMA and waits 20 ms; pass 3's
+                         // odd lanes count their line copies as late
 };
 
 // One batched launch of a pass over several realisations that share the
