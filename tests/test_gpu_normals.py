@@ -1,0 +1,79 @@
+"""The generator's draws on chosen words: the device functions of
+scarl_common.cuh compiled with the package's flags and evaluated at the edges of
+their ranges and on random words."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import scarl_b200.build as B
+
+pytestmark = pytest.mark.gpu
+
+SRC = r"""
+#include "scarl_common.cuh"
+using namespace scarl;
+// per word pair: the FP32 pair, the argument of its square root
+__global__ void k32(const uint32_t* a, const uint32_t* b, int n, float* o) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const float2 p = Normals<float>::from(a[i], b[i]);
+  o[3 * i] = p.x;
+  o[3 * i + 1] = p.y;
+  o[3 * i + 2] = -1.38629436111989061883f * lg2_ftz(__fmaf_rn((float)a[i], 0x1p-32f, 0x1p-33f));
+}
+template <class K, class O> static int run(K k, const uint32_t* a, const uint32_t* b, int n, int w, O* out) {
+  uint32_t *da, *db;
+  O* d;
+  if (cudaMalloc(&da, 4 * (size_t)n) || cudaMalloc(&db, 4 * (size_t)n) || cudaMalloc(&d, sizeof(O) * (size_t)n * w)) return 1;
+  cudaMemcpy(da, a, 4 * (size_t)n, cudaMemcpyHostToDevice);
+  cudaMemcpy(db, b, 4 * (size_t)n, cudaMemcpyHostToDevice);
+  k<<<(n + 255) / 256, 256>>>(da, db, n, d);
+  const int rc = cudaMemcpy(out, d, sizeof(O) * (size_t)n * w, cudaMemcpyDeviceToHost);
+  cudaFree(da), cudaFree(db), cudaFree(d);
+  return rc;
+}
+extern "C" int draw32(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(k32, a, b, n, 3, o); }
+"""
+
+
+@pytest.fixture(scope="module")
+def dev(tmp_path_factory):
+    d = tmp_path_factory.mktemp("draws")
+    (d / "draws.cu").write_text(SRC)
+    so = str(d / "draws.so")
+    subprocess.check_call([B._nvcc()] + B.ARCH + B.COMMON + ["-shared", "-cudart", "static", str(d / "draws.cu"), "-o", so])
+    return C.CDLL(so)
+
+
+def call(fn, a, b, w, dt):
+    a, b = np.ascontiguousarray(a, np.uint32), np.ascontiguousarray(b, np.uint32)
+    out = np.empty((a.size, w), dt)
+    assert fn(C.c_void_p(a.ctypes.data), C.c_void_p(b.ctypes.data), a.size, C.c_void_p(out.ctypes.data)) == 0
+    return out
+
+
+def words():
+    """Both ends, the edges of the 64ths of every octave, the neighbourhoods of
+    the multiples of an eighth turn, and random words."""
+    e = [np.arange(4096), 0xFFFFFFFF - np.arange(1 << 16)]
+    edges = np.array([(64 + i) << s for s in range(27) for i in range(64)], dtype=np.int64)
+    e += [edges + d for d in (-1, 0, 1)]
+    e += [np.arange(-2048, 2048) + (k << 29) for k in range(8)]
+    e.append(np.random.default_rng(9).integers(0, 1 << 32, 1 << 20))
+    return (np.concatenate(e).astype(np.int64) & 0xFFFFFFFF).astype(np.uint32)
+
+
+def test_fp32_radius(dev):
+    """At b = 0 the phase is -pi up to 2^-32, whose cosine rounds to -1: the first
+    component is the radius sqrt(-2 ln u1).  Its root is within half a unit in the
+    last place and 2^-44 relative (2^-20 units; 1e-5 with the double rounding of
+    the comparison)."""
+    a = words()
+    o = call(dev.draw32, a, np.zeros_like(a), 3, np.float32)
+    assert np.isfinite(o).all()
+    r, ref = o[:, 0], np.sqrt(np.abs(o[:, 2]).astype(np.float64))
+    ulp = np.spacing(np.maximum(ref, 2.0 ** -60).astype(np.float32)).astype(np.float64)
+    assert (np.abs(r - ref) <= (0.5 + 1e-5) * ulp).all()
