@@ -74,20 +74,6 @@ struct TcCfg {
 
 constexpr uint64_t kWaitNs = 1000000000ull;  // 1 s per tensor-core wait
 
-// The canonical Box-Muller pair of Normals<float> (u1 = (a + 1/2) 2^-32,
-// u2 = (b + 1/2) 2^-32, r (cos 2 pi u2, sin 2 pi u2), r = sqrt(-2 ln u1)) at
-// the split path's accuracy: the phase 2 pi (u2 - 1/2) from the top 23 bits of
-// b as the mantissa of m in [1, 2), by one fused multiply-add and without a
-// conversion (phase error under 2^-21, far below the 2^-17 of the BF16 split).
-__device__ __forceinline__ float2 split_normals(uint32_t a, uint32_t b) {
-  constexpr float k2Pi = 6.28318530717958647692f;
-  const float u1 = __fmaf_rn((float)a, 0x1p-32f, 0x1p-33f);
-  const float r = sqrt_ftz(-1.38629436111989061883f * lg2_ftz(u1));
-  float s, c;
-  sincos_ftz(__fmaf_rn(__uint_as_float(0x3F800000u | (b >> 9)), k2Pi, (-1.5f + 0x1p-24f) * k2Pi), &s, &c);
-  return make_float2(-r * c, -r * s);
-}
-
 // b^e for b >= 1 as 2^(e log2 b) on the hardware approximations (lg2.approx,
 // ex2.approx): relative error a few 2^-22 for the exponents of the Matern
 // amplitude (e = -(nu + 3/2) / 2), far below the 2^-17 of the BF16 split.

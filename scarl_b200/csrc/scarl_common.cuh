@@ -246,15 +246,19 @@ __device__ __forceinline__ void sincos_ftz(float x, float* s, float* c) {
   asm("sin.approx.ftz.f32 %0, %1;" : "=f"(*s) : "f"(x));
   asm("cos.approx.ftz.f32 %0, %1;" : "=f"(*c) : "f"(x));
 }
+// -2 ln u for 0 < u <= 1.  The hardware logarithm's error is absolute, 2^-22 for
+// u above 1/2, so its sign near u = 1 is not the specification's to promise: the
+// magnitude is taken (it costs nothing), and no root sees a negative.
+__device__ __forceinline__ float neg2ln(float u) { return fabsf(-1.38629436111989061883f * lg2_ftz(u)); }
 template <> struct Normals<float> {
-  // Single precision, hardware logarithm, sine and cosine: u1 is formed with one rounding (relative error 2^-24, so small
-  // u1 keep their digits).  The phase
+  // Single precision, hardware logarithm, sine and cosine: u1 is formed with
+  // one rounding (relative error 2^-24, so small u1 keep their digits).  The phase
   // 2 pi (u2 - 1/2) in (-pi, pi), where the hardware sine is accurate, comes
   // from the signed word b - 2^31 by one fused multiply-add: relative error
   // 2^-24 of the reduced phase, not of u2.  The half-turn is the sign.
   static __device__ __forceinline__ float2 from(uint32_t a, uint32_t b) {
     const float u1 = __fmaf_rn((float)a, 0x1p-32f, 0x1p-33f);
-    const float r = sqrt_newton(-1.38629436111989061883f * lg2_ftz(u1));  // -2 ln 2 lg2 u1 >= 0
+    const float r = sqrt_newton(neg2ln(u1));
     const float ph = __fmaf_rn((float)(int32_t)(b ^ 0x80000000u), 6.28318530717958647692f * 0x1p-32f,
                                6.28318530717958647692f * 0x1p-33f);
     float s, c;
@@ -262,6 +266,20 @@ template <> struct Normals<float> {
     return make_float2(-r * c, -r * s);
   }
 };
+
+// The canonical Box-Muller pair of Normals<float> (u1 = (a + 1/2) 2^-32,
+// u2 = (b + 1/2) 2^-32, r (cos 2 pi u2, sin 2 pi u2), r = sqrt(-2 ln u1)) at
+// the split path's accuracy: the phase 2 pi (u2 - 1/2) from the top 23 bits of
+// b as the mantissa of m in [1, 2), by one fused multiply-add and without a
+// conversion (phase error under 2^-21, far below the 2^-17 of the BF16 split).
+__device__ __forceinline__ float2 split_normals(uint32_t a, uint32_t b) {
+  constexpr float k2Pi = 6.28318530717958647692f;
+  const float u1 = __fmaf_rn((float)a, 0x1p-32f, 0x1p-33f);
+  const float r = sqrt_ftz(neg2ln(u1));
+  float s, c;
+  sincos_ftz(__fmaf_rn(__uint_as_float(0x3F800000u | (b >> 9)), k2Pi, (-1.5f + 0x1p-24f) * k2Pi), &s, &c);
+  return make_float2(-r * c, -r * s);
+}
 
 // ---------------------------------------------------------------------------
 // Park-Miller (16807, 2^31-1): state after n steps from s, s in [0, 2^31-1).

@@ -24,6 +24,21 @@ __global__ void k32(const uint32_t* a, const uint32_t* b, int n, float* o) {
   o[3 * i + 1] = p.y;
   o[3 * i + 2] = -1.38629436111989061883f * lg2_ftz(__fmaf_rn((float)a[i], 0x1p-32f, 0x1p-33f));
 }
+// the split path's pair
+__global__ void ksplit(const uint32_t* a, const uint32_t* b, int n, float* o) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const float2 p = split_normals(a[i], b[i]);
+  o[2 * i] = p.x;
+  o[2 * i + 1] = p.y;
+}
+// word a as the bits of u: lg2 u and -2 ln u
+__global__ void klg2(const uint32_t* a, const uint32_t*, int n, float* o) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  o[2 * i] = lg2_ftz(__uint_as_float(a[i]));
+  o[2 * i + 1] = neg2ln(__uint_as_float(a[i]));
+}
 template <class K, class O> static int run(K k, const uint32_t* a, const uint32_t* b, int n, int w, O* out) {
   uint32_t *da, *db;
   O* d;
@@ -35,6 +50,8 @@ template <class K, class O> static int run(K k, const uint32_t* a, const uint32_
   cudaFree(da), cudaFree(db), cudaFree(d);
   return rc;
 }
+extern "C" int split(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(ksplit, a, b, n, 2, o); }
+extern "C" int lg2(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(klg2, a, b, n, 2, o); }
 extern "C" int draw32(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(k32, a, b, n, 3, o); }
 """
 
@@ -77,3 +94,17 @@ def test_fp32_radius(dev):
     r, ref = o[:, 0], np.sqrt(np.abs(o[:, 2]).astype(np.float64))
     ulp = np.spacing(np.maximum(ref, 2.0 ** -60).astype(np.float32)).astype(np.float64)
     assert (np.abs(r - ref) <= (0.5 + 1e-5) * ulp).all()
+
+
+def test_log_keeps_its_sign_up_to_one(dev):
+    """Every u from 1 - 2^-7 to 1, and the powers of two down to 2^-33: the
+    logarithm is never positive, the argument of the radius never negative, and
+    the draws at u = 1 are finite."""
+    one = np.float32(1).view(np.uint32)
+    bits = np.concatenate([one - np.arange(1 << 17), one - (np.arange(34) << 23)]).astype(np.uint32)
+    o = call(dev.lg2, bits, bits, 2, np.float32)
+    assert (o[:, 0] <= 0).all() and (o[:, 1] >= 0).all() and not np.signbit(o[:, 1]).any()
+    a = np.full(4, 0xFFFFFFFF, np.uint32)
+    b = np.arange(4, dtype=np.uint32) << 30
+    for f, w in ((dev.draw32, 3), (dev.split, 2)):
+        assert np.isfinite(call(f, a, b, w, np.float32)).all()
