@@ -270,14 +270,19 @@ template <> struct Normals<float> {
 // The canonical Box-Muller pair of Normals<float> (u1 = (a + 1/2) 2^-32,
 // u2 = (b + 1/2) 2^-32, r (cos 2 pi u2, sin 2 pi u2), r = sqrt(-2 ln u1)) at
 // the split path's accuracy: the phase 2 pi (u2 - 1/2) from the top 23 bits of
-// b as the mantissa of m in [1, 2), by one fused multiply-add and without a
-// conversion (phase error under 2^-21, far below the 2^-17 of the BF16 split).
-__device__ __forceinline__ float2 split_normals(uint32_t a, uint32_t b) {
+// b as the mantissa of m in [1, 2), without a conversion; m - 3/2 is exact, the
+// half step comes in with the product.  Phase error up to 5.8e-7 (the 23 bits
+// 3.7e-7, the rounding 1.2e-7, 2 pi as a float 0.9e-7) and 0 on average, far below
+// the 2^-17 of the BF16 split.
+__device__ __forceinline__ float split_phase(uint32_t b) {
   constexpr float k2Pi = 6.28318530717958647692f;
+  return __fmaf_rn(__uint_as_float(0x3F800000u | (b >> 9)) - 1.5f, k2Pi, 0x1p-24f * k2Pi);
+}
+__device__ __forceinline__ float2 split_normals(uint32_t a, uint32_t b) {
   const float u1 = __fmaf_rn((float)a, 0x1p-32f, 0x1p-33f);
   const float r = sqrt_ftz(neg2ln(u1));
   float s, c;
-  sincos_ftz(__fmaf_rn(__uint_as_float(0x3F800000u | (b >> 9)), k2Pi, (-1.5f + 0x1p-24f) * k2Pi), &s, &c);
+  sincos_ftz(split_phase(b), &s, &c);
   return make_float2(-r * c, -r * s);
 }
 
