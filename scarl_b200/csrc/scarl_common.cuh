@@ -126,70 +126,94 @@ template <typename T> struct Normals;
 // "Table-driven implementation of the logarithm function in IEEE floating-point
 // arithmetic", ACM TOMS 16, 1990, with 64 intervals), sine and cosine by their
 // Taylor series after an exact integer reduction to an eighth turn.  Measured
-// against extended precision over 4 M words and the ends of every interval: ln
-// within 2.3 x 2^-53 max(1, |ln u|), the pair within 1.7e-16; the FP64 field's
-// error is the same 9e-16.  With the general log and sincospi, their special
-// cases and their conversions, pass 1 of four 256 x 224 x 256 grids took 365 us,
-// with these 324.
+// against extended precision over 4 M random words, both ends and every
+// interval's and octant's edges: ln u within 1.13e-16 of its own size (rms
+// 4.7e-17), cosine and sine within 1.2e-16 (rms 2.8e-17); log has the same,
+// sincospi 1.3e-16 and 3.2e-17.  A sample of four 256 x 224 x 256 grids takes 684
+// us; 711 with log and sincospi, their special cases and their conversions.
 //
-// Interval i of [1, 2): {c, -ln c}, c the rounded inverse of its middle; the
-// last one has c = 1/2 and ln 2, so that u near 1 keeps its digits.
+// u = f / 2 2^k with f in [1, 2), k <= 0: k ln 2 and the logarithm of f / 2 are both
+// negative, so that nothing cancels near u = 1.  Interval i of f: {c, -ln 2c}, 1 / c
+// about its middle and c of 20 bits (f c - 1 is exact for the 33 bits of f), the
+// last one c = 1/2; -ln 2c in two parts, the first a multiple of 2^-47 like that of
+// ln 2, so that the sum k ln 2 - ln 2c of the first parts is exact.
 __device__ const double2 kLogTab[64] = {
-    {0x1.fc07f01fc07f0p-1, 0x1.fe02a6b106799p-8}, {0x1.f44659e4a4271p-1, 0x1.7b91b07d5b126p-6},
-    {0x1.ecc07b301ecc0p-1, 0x1.39e87b9febd68p-5}, {0x1.e573ac901e574p-1, 0x1.b42dd711971b9p-5},
-    {0x1.de5d6e3f8868ap-1, 0x1.16536eea37ae3p-4}, {0x1.d77b654b82c34p-1, 0x1.51b073f06183cp-4},
-    {0x1.d0cb58f6ec074p-1, 0x1.8c345d6319b23p-4}, {0x1.ca4b3055ee191p-1, 0x1.c5e548f5bc743p-4},
-    {0x1.c3f8f01c3f8f0p-1, 0x1.fec9131dbeabcp-4}, {0x1.bdd2b899406f7p-1, 0x1.1b72ad52f67a2p-3},
-    {0x1.b7d6c3dda338bp-1, 0x1.371fc201e8f75p-3}, {0x1.b2036406c80d9p-1, 0x1.526e5e3a1b438p-3},
-    {0x1.ac5701ac5701bp-1, 0x1.6d60fe719d21bp-3}, {0x1.a6d01a6d01a6dp-1, 0x1.87fa06520c911p-3},
-    {0x1.a16d3f97a4b02p-1, 0x1.a23bc1fe2b561p-3}, {0x1.9c2d14ee4a102p-1, 0x1.bc286742d8cd4p-3},
-    {0x1.970e4f80cb872p-1, 0x1.d5c216b4fbb94p-3}, {0x1.920fb49d0e229p-1, 0x1.ef0adcbdc5935p-3},
-    {0x1.8d3018d3018d3p-1, 0x1.0402594b4d041p-2}, {0x1.886e5f0abb04ap-1, 0x1.1058bf9ae4ad4p-2},
-    {0x1.83c977ab2beddp-1, 0x1.1c898c16999fbp-2}, {0x1.7f405fd017f40p-1, 0x1.2895a13de86a4p-2},
-    {0x1.7ad2208e0ecc3p-1, 0x1.347dd9a987d56p-2}, {0x1.767dce434a9b1p-1, 0x1.404308686a7e4p-2},
-    {0x1.724287f46debcp-1, 0x1.4be5f957778a1p-2}, {0x1.6e1f76b4337c7p-1, 0x1.5767717455a6cp-2},
-    {0x1.6a13cd1537290p-1, 0x1.62c82f2b9c796p-2}, {0x1.661ec6a5122f9p-1, 0x1.6e08eaa2ba1e4p-2},
-    {0x1.623fa77016240p-1, 0x1.792a55fdd47a1p-2}, {0x1.5e75bb8d015e7p-1, 0x1.842d1da1e8b18p-2},
-    {0x1.5ac056b015ac0p-1, 0x1.8f11e873662c8p-2}, {0x1.571ed3c506b3ap-1, 0x1.99d958117e08ap-2},
-    {0x1.5390948f40febp-1, 0x1.a484090e5bb09p-2}, {0x1.5015015015015p-1, 0x1.af1293247786bp-2},
-    {0x1.4cab88725af6ep-1, 0x1.b9858969310fdp-2}, {0x1.49539e3b2d067p-1, 0x1.c3dd7a7cdad4dp-2},
-    {0x1.460cbc7f5cf9ap-1, 0x1.ce1af0b85f3ecp-2}, {0x1.42d6625d51f87p-1, 0x1.d83e7258a2f3ep-2},
-    {0x1.3fb013fb013fbp-1, 0x1.e24881a7c6c26p-2}, {0x1.3c995a47babe7p-1, 0x1.ec399d2468cc1p-2},
-    {0x1.3991c2c187f63p-1, 0x1.f6123fa7028adp-2}, {0x1.3698df3de0748p-1, 0x1.ffd2e0857f497p-2},
-    {0x1.33ae45b57bcb2p-1, 0x1.04bdf9da926d2p-1}, {0x1.30d190130d190p-1, 0x1.0986f4f573521p-1},
-    {0x1.2e025c04b8097p-1, 0x1.0e44985d1cc8cp-1}, {0x1.2b404ad012b40p-1, 0x1.12f719593efbdp-1},
-    {0x1.288b01288b013p-1, 0x1.179eabbd899a0p-1}, {0x1.25e22708092f1p-1, 0x1.1c3b81f713c25p-1},
-    {0x1.23456789abcdfp-1, 0x1.20cdcd192ab6ep-1}, {0x1.20b470c67c0d9p-1, 0x1.2555bce98f7cap-1},
-    {0x1.1e2ef3b3fb874p-1, 0x1.29d37fec2b08bp-1}, {0x1.1bb4a4046ed29p-1, 0x1.2e47436e40268p-1},
-    {0x1.19453808ca29cp-1, 0x1.32b1339121d71p-1}, {0x1.16e0689427379p-1, 0x1.37117b54747b6p-1},
-    {0x1.1485f0e0acd3bp-1, 0x1.3b68449fffc23p-1}, {0x1.12358e75d3033p-1, 0x1.3fb5b84d16f43p-1},
-    {0x1.0fef010fef011p-1, 0x1.43f9fe2f9ce67p-1}, {0x1.0db20a88f4696p-1, 0x1.48353d1ea88dfp-1},
-    {0x1.0b7e6ec259dc8p-1, 0x1.4c679afccee39p-1}, {0x1.0953f39010954p-1, 0x1.50913cc01686bp-1},
-    {0x1.073260a47f7c6p-1, 0x1.54b2467999498p-1}, {0x1.05197f7d73404p-1, 0x1.58cadb5cd7989p-1},
-    {0x1.03091b51f5e1ap-1, 0x1.5cdb1dc6c1765p-1}, {0x1.0000000000000p-1, 0x1.62e42fefa39efp-1}};
+    {0x1.fc08000000000p-1, -0x1.5ee83aa241540p-1}, {0x1.f446600000000p-1, -0x1.5707a8abb8bc0p-1},
+    {0x1.ecc0800000000p-1, -0x1.4f45ad35a4dc0p-1}, {0x1.e573a00000000p-1, -0x1.47a1453e8a000p-1},
+    {0x1.de5d600000000p-1, -0x1.4019b2d25c700p-1}, {0x1.d77b600000000p-1, -0x1.38ae1bb197680p-1},
+    {0x1.d0cb600000000p-1, -0x1.315dac0340580p-1}, {0x1.ca4b400000000p-1, -0x1.2a279850ebc40p-1},
+    {0x1.c3f9000000000p-1, -0x1.230b1f8beb780p-1}, {0x1.bdd2c00000000p-1, -0x1.1c078d1ae5f00p-1},
+    {0x1.b7d6c00000000p-1, -0x1.151c3aef295c0p-1}, {0x1.b203600000000p-1, -0x1.0e4893a11cc80p-1},
+    {0x1.ac57000000000p-1, -0x1.078bee533c540p-1}, {0x1.a6d0200000000p-1, -0x1.00e5b51b20700p-1},
+    {0x1.a16d400000000p-1, -0x1.f4aa7fe031900p-2}, {0x1.9c2d200000000p-1, -0x1.e7b447bdda780p-2},
+    {0x1.970e400000000p-1, -0x1.dae72d84c8a00p-2}, {0x1.920fc00000000p-1, -0x1.ce430e8064080p-2},
+    {0x1.8d30200000000p-1, -0x1.c1c61913fa100p-2}, {0x1.886e600000000p-1, -0x1.b56fa2c462900p-2},
+    {0x1.83c9800000000p-1, -0x1.a93ee9c8ad600p-2}, {0x1.7f40600000000p-1, -0x1.9d32bf215ed00p-2},
+    {0x1.7ad2200000000p-1, -0x1.914a84b5bf680p-2}, {0x1.767dc00000000p-1, -0x1.85853076dc000p-2},
+    {0x1.7242800000000p-1, -0x1.79e25087cf780p-2}, {0x1.6e1f800000000p-1, -0x1.6e61086af1400p-2},
+    {0x1.6a13c00000000p-1, -0x1.63000bb3aa180p-2}, {0x1.661ec00000000p-1, -0x1.57bf623c8cf00p-2},
+    {0x1.623fa00000000p-1, -0x1.4c9df46172880p-2}, {0x1.5e75c00000000p-1, -0x1.419b4f3d5e780p-2},
+    {0x1.5ac0600000000p-1, -0x1.36b692ebe0b00p-2}, {0x1.571ee00000000p-1, -0x1.2bef2c4dc8900p-2},
+    {0x1.5390a00000000p-1, -0x1.21447950eaf80p-2}, {0x1.5015000000000p-1, -0x1.16b5c8bacfb80p-2},
+    {0x1.4cab800000000p-1, -0x1.0c42bc7615d80p-2}, {0x1.4953a00000000p-1, -0x1.01eaeae26c680p-2},
+    {0x1.460cc00000000p-1, -0x1.ef5af44dcfe00p-3}, {0x1.42d6600000000p-1, -0x1.db13cc0d48800p-3},
+    {0x1.3fb0200000000p-1, -0x1.c700096eff800p-3}, {0x1.3c99600000000p-1, -0x1.b31daa75bc900p-3},
+    {0x1.3991c00000000p-1, -0x1.9f6c2e7089500p-3}, {0x1.3698e00000000p-1, -0x1.8beb03b38fe00p-3},
+    {0x1.33ae400000000p-1, -0x1.7898b25444700p-3}, {0x1.30d1a00000000p-1, -0x1.657556e8be700p-3},
+    {0x1.2e02600000000p-1, -0x1.527e794a1b300p-3}, {0x1.2b40400000000p-1, -0x1.3fb4105991300p-3},
+    {0x1.288b000000000p-1, -0x1.2d1608c868100p-3}, {0x1.25e2200000000p-1, -0x1.1aa286e23ee00p-3},
+    {0x1.2345600000000p-1, -0x1.08595659e2f00p-3}, {0x1.20b4800000000p-1, -0x1.ec7470309b600p-4},
+    {0x1.1e2f000000000p-1, -0x1.c886301bc0e00p-4}, {0x1.1bb4a00000000p-1, -0x1.a4e72a0b1b600p-4},
+    {0x1.1945400000000p-1, -0x1.819856f40ca00p-4}, {0x1.16e0600000000p-1, -0x1.5e9526d977200p-4},
+    {0x1.1486000000000p-1, -0x1.3be03a7d18c00p-4}, {0x1.1235800000000p-1, -0x1.1972e5145fa00p-4},
+    {0x1.0fef000000000p-1, -0x1.eea2fc006b800p-5}, {0x1.0db2000000000p-1, -0x1.aaeded0faac00p-5},
+    {0x1.0b7e600000000p-1, -0x1.67c78b2d3f400p-5}, {0x1.0954000000000p-1, -0x1.2530b2f8c8800p-5},
+    {0x1.0732600000000p-1, -0x1.c63d06c14a800p-6}, {0x1.0519800000000p-1, -0x1.432ab25981000p-6},
+    {0x1.0309200000000p-1, -0x1.8246da3885000p-7}, {0x1.0000000000000p-1, 0x0.0p+0}};
+__device__ const double kLogTail[64] = {
+    0x1.fdc69dd06becep-49, -0x1.4406284a2c39fp-50, 0x1.58a2c6521cc72p-50, -0x1.509444d8f0e83p-49,
+    0x1.e4f4b0fa46764p-50, 0x1.cf7acb2d14713p-49, -0x1.ad6c61296748cp-49, 0x1.1692ce596f827p-52,
+    -0x1.f814749099b49p-51, 0x1.9d4c511ce7b43p-49, -0x1.26855d451aa72p-53, -0x1.c32feb46d8ee7p-51,
+    -0x1.812241434b51fp-49, 0x1.65d1a5773e100p-50, -0x1.56f2b7834ff05p-49, -0x1.5ac214be4fbf7p-51,
+    -0x1.9de6e5a9bda4cp-49, -0x1.8a102e5b6643dp-49, 0x1.ddfcf88b283d2p-51, 0x1.96d6914488afap-53,
+    -0x1.b6f39c7ccc1ecp-50, -0x1.d461ef2f94a4ep-49, -0x1.452b441f3e0d2p-52, -0x1.8ad99296cbc6dp-50,
+    0x1.4e0cffb653f06p-51, -0x1.50b37526689c1p-49, -0x1.73b412573211bp-50, -0x1.46f6afbbf4ce1p-49,
+    -0x1.f6ecfadda0cb0p-50, 0x1.5bc8b7e475979p-51, -0x1.7367b11b0cdc2p-49, 0x1.4e07764f6682ap-50,
+    -0x1.efcad2851f5b3p-52, 0x1.65320905942a0p-49, -0x1.b114be4f242d6p-50, 0x1.5c46088749fbfp-49,
+    -0x1.deee1199c01dfp-55, -0x1.7cd504854fc53p-49, -0x1.1e73f9bed46d4p-49, 0x1.c58c46db8fe82p-51,
+    -0x1.009ac19b02d9ap-50, -0x1.ccaad56f5f767p-49, 0x1.8610ff769a574p-50, 0x1.fc342ec67c9a8p-49,
+    0x1.301700f5827a4p-49, -0x1.9e2571f311bbdp-49, 0x1.8a4cdca3d82f6p-53, 0x1.b8e4a9ef7dc19p-50,
+    -0x1.b10e70e60b318p-52, 0x1.891e9a1afee90p-59, -0x1.46d53dafe5901p-49, 0x1.695b9c2559e62p-50,
+    0x1.5f8f872d61247p-50, -0x1.92f87e0ddb5f3p-49, -0x1.90cb9660b2485p-50, -0x1.1b388364410b8p-50,
+    0x1.089f2939f3141p-50, -0x1.f82f3521ebf6cp-50, 0x1.5e328e632292ap-52, -0x1.f4fb010c6fd4fp-52,
+    -0x1.14c63f750847cp-49, 0x1.dfb19b491cab3p-49, 0x1.72ef3101439fep-50, 0x0.0p+0};
 template <> struct Normals<double> {
   // ln((a + 1/2) 2^-32)
   static __device__ __forceinline__ double ln_u(uint32_t a) {
     const double x = __hiloint2double(0x43300000, (int)a) - (0x1p52 - 0.5);  // a + 1/2, exact
-    const int hi = __double2hiint(x);
+    const int hi = __double2hiint(x), i = (hi >> 14) & 63;
     const double f = __hiloint2double((hi & 0xFFFFF) | 0x3FF00000, __double2loint(x));  // x = f 2^e
-    const double2 t = __ldg(&kLogTab[(hi >> 14) & 63]);
-    const double k = __hiloint2double(0x43300000, (hi >> 20) - 1023 - 32 + 64) - (0x1p52 + 64.0);  // e - 32, exact
-    const double r = fma(f, t.x, -1.0);  // |r| < 2^-7
+    const double2 t = __ldg(&kLogTab[i]);
+    const double k = __hiloint2double(0x43300000, (hi >> 20) - 1023 - 31 + 64) - (0x1p52 + 64.0);  // e - 31, exact
+    const double r = fma(f, t.x, -1.0);  // |r| <= 2^-7, exact
     double q = fma(r, -1.0 / 8.0, 1.0 / 7.0);
     q = fma(q, r, -1.0 / 6.0);
     q = fma(q, r, 1.0 / 5.0);
     q = fma(q, r, -1.0 / 4.0);
     q = fma(q, r, 1.0 / 3.0);
     q = fma(q, r, -0.5);
-    return fma(k, 0x1.62e42fefa39efp-1, t.y) + fma(r * r, q, r);
+    const double s = fma(k, 0x1.62e42fefa3a00p-1, t.y);  // exact; 0 or larger than r
+    const double w = s + r, e = r - (w - s);          // e: what w's rounding lost
+    return w + fma(r * r, q, e + fma(k, -0x1.0ca86c3898d00p-49, __ldg(&kLogTail[i])));
   }
   // cos and sin of 2 pi (b + 1/2) 2^-32
   static __device__ __forceinline__ void circle(uint32_t b, double* c, double* s) {
     const uint32_t q = (b + 0x20000000u) >> 30;  // quarter turns
     const uint32_t d = b - (q << 30);            // as signed: [-2^29, 2^29)
-    constexpr double kStep = 6.283185307179586476925 * 0x1p-32;
-    const double p = fma(__hiloint2double(0x43300000, (int)(d ^ 0x80000000u)) - (0x1p52 + 0x1p31), kStep, 0.5 * kStep);
+    // the phase p + pe: 2 pi 2^-32 in two parts
+    constexpr double kStep = 6.283185307179586476925 * 0x1p-32, kStepTail = 2.4492935982947064e-16 * 0x1p-32;
+    const double y = __hiloint2double(0x43300000, (int)(d ^ 0x80000000u)) - (0x1p52 + 0x1p31) + 0.5;  // exact
+    const double p = y * kStep, pe = fma(y, kStepTail, fma(y, kStep, -p));
     const double z = p * p;
     double u = fma(z, -1.0 / 1307674368000.0, 1.0 / 6227020800.0);
     u = fma(u, z, -1.0 / 39916800.0);
@@ -197,15 +221,15 @@ template <> struct Normals<double> {
     u = fma(u, z, -1.0 / 5040.0);
     u = fma(u, z, 1.0 / 120.0);
     u = fma(u, z, -1.0 / 6.0);
-    const double sn = fma(p * z, u, p);
+    const double sn = p + fma(p * z, u, pe);
     double v = fma(z, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);
     v = fma(v, z, 1.0 / 479001600.0);
     v = fma(v, z, -1.0 / 3628800.0);
     v = fma(v, z, 1.0 / 40320.0);
     v = fma(v, z, -1.0 / 720.0);
     v = fma(v, z, 1.0 / 24.0);
-    v = fma(v, z, -0.5);
-    const double cs = fma(v, z, 1.0);
+    const double h = fma(z, -0.5, 1.0), ht = fma(z, -0.5, 1.0 - h);  // 1 - z / 2 and what its rounding lost
+    const double cs = h + fma(z * z, v, fma(-p, pe, ht));
     const double cq = (q & 1) ? sn : cs, sq = (q & 1) ? cs : sn;  // q = 1: (-s, c), 2: (-c, -s), 3: (s, -c)
     *c = __hiloint2double(__double2hiint(cq) ^ (int)(((q + 1) & 2) << 30), __double2loint(cq));
     *s = __hiloint2double(__double2hiint(sq) ^ (int)((q & 2) << 30), __double2loint(sq));

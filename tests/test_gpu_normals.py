@@ -43,6 +43,13 @@ __global__ void klg2(const uint32_t* a, const uint32_t*, int n, float* o) {
   o[2 * i] = lg2_ftz(__uint_as_float(a[i]));
   o[2 * i + 1] = neg2ln(__uint_as_float(a[i]));
 }
+// FP64: ln((a + 1/2) 2^-32), cosine and sine of 2 pi (b + 1/2) 2^-32
+__global__ void k64(const uint32_t* a, const uint32_t* b, int n, double* o) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  o[3 * i] = Normals<double>::ln_u(a[i]);
+  Normals<double>::circle(b[i], o + 3 * i + 1, o + 3 * i + 2);
+}
 template <class K, class O> static int run(K k, const uint32_t* a, const uint32_t* b, int n, int w, O* out) {
   uint32_t *da, *db;
   O* d;
@@ -56,6 +63,7 @@ template <class K, class O> static int run(K k, const uint32_t* a, const uint32_
 }
 extern "C" int split(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(ksplit, a, b, n, 2, o); }
 extern "C" int phase(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(kphase, a, b, n, 1, o); }
+extern "C" int draw64(const uint32_t* a, const uint32_t* b, int n, double* o) { return run(k64, a, b, n, 3, o); }
 extern "C" int lg2(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(klg2, a, b, n, 2, o); }
 extern "C" int draw32(const uint32_t* a, const uint32_t* b, int n, float* o) { return run(k32, a, b, n, 3, o); }
 """
@@ -125,3 +133,25 @@ def test_split_phase(dev):
     e = call(dev.phase, b, b, 1, np.float32)[:, 0] - ref
     assert np.abs(e).max() <= 5.9e-7
     assert abs(e[-(1 << 20):].mean()) <= 3e-9
+
+
+def test_fp64_log_and_circle(dev):
+    """The FP64 logarithm by table and the sine and cosine by series against
+    extended precision.  Logarithm: half a unit in the last place of the result
+    and 2^-5 of that for the terms added to it (at most 2^-8 of the result, three
+    roundings), every table entry among the arguments.  Sine and cosine, absolute:
+    half a unit below 1 (2^-54), the rounding of z / 2 (2^-55), 4.6e-17 from the
+    series' first missing term and 0.6e-17 from the rest."""
+    w = words()
+    o = call(dev.draw64, w, w, 3, np.float64)
+    one = np.longdouble(1)
+    u = (w.astype(np.longdouble) + one / 2) * one / 2 ** 32
+    ln = np.log(u)
+    assert (np.abs(o[:, 0] - ln) <= (1 + 2.0 ** -5) * 2.0 ** -53 * np.abs(ln)).all()
+    q = ((w + np.uint32(1 << 29)) >> 30).astype(np.int64)
+    pi2 = 8 * np.arctan(one)
+    p = ((w - (q.astype(np.uint32) << 30)).view(np.int32).astype(np.longdouble) + one / 2) / 2 ** 32 * pi2
+    c, s = np.cos(p), np.sin(p)
+    c, s = np.choose(q & 3, [c, -s, -c, s]), np.choose(q & 3, [s, c, -s, -c])
+    tol = 2.0 ** -54 + 2.0 ** -55 + 4.6e-17 + 0.6e-17
+    assert (np.abs(o[:, 1] - c) <= tol).all() and (np.abs(o[:, 2] - s) <= tol).all()
