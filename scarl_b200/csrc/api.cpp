@@ -151,6 +151,12 @@ constexpr size_t kRingMin = (size_t)8 << 20;
 // (83 MB 84 against 115) and ends (252 MB 254 against 244, 941 MB 869 against 583),
 // where one tile fills the GPU and saves the tiles' round trip through memory
 constexpr size_t kDctBatch = (size_t)64 << 20;
+// a cosine matrix is kept up to the first size (lengths to 8192 over half the
+// inputs, 5793 over all), all of them together up to the second; longer axes form
+// their cosines in the kernel (8300 points along x / y / z by 64 x 64: 2.6 / 4.9 /
+// 9.4 ms against 1.5 / 2.6 / 5.1 with the matrix, which grows with the square of
+// the length: 3.2 GB at 40000)
+constexpr size_t kDctTab = (size_t)128 << 20, kDctTabs = (size_t)384 << 20;
 
 }  // namespace
 
@@ -177,7 +183,8 @@ struct scarl_ctx {
   HostPool* hpool = nullptr;
   std::map<std::string, PaddedPlan> plans;
   std::map<long long, Buf> twiddles;
-  std::map<std::pair<int, int>, Buf> dct_tabs;  // (length, inputs) -> folded cosines
+  std::map<std::pair<int, int>, Buf> dct_tabs;  // (length, inputs) -> folded cosines; inputs 0: the roots
+  std::vector<std::pair<int, int>> dct_held;    // tables of the call in progress
   bool profile = false;
   long long launches = 0;
   unsigned long long h2d = 0, d2h = 0;
@@ -215,19 +222,46 @@ int fail(scarl_ctx* c, int code, const std::string& m) {
     if (r_ != SCARL_OK) return r_;   \
   } while (0)
 
+void release(scarl_ctx* ctx, Buf& b) {
+  if (b.p) {
+    cudaFree(b.p);
+    ctx->used -= b.n;
+  }
+  b.p = nullptr;
+  b.n = 0;
+}
+
+// Frees the literal generator's cosine tables except those of the call in
+// progress (cudaFree waits for kernels that read them); true if any was.
+bool drop_dct_tabs(scarl_ctx* ctx) {
+  bool any = false;
+  for (auto it = ctx->dct_tabs.begin(); it != ctx->dct_tabs.end();) {
+    if (std::find(ctx->dct_held.begin(), ctx->dct_held.end(), it->first) != ctx->dct_held.end()) {
+      ++it;
+      continue;
+    }
+    release(ctx, it->second);
+    it = ctx->dct_tabs.erase(it);
+    any = true;
+  }
+  return any;
+}
+
+// Grows b to the given size.  The cosine tables, which can be formed again, give
+// way where the budget or the device has no room.
 int ensure(scarl_ctx* ctx, Buf& b, size_t bytes) {
   if (bytes == 0) bytes = 16;
   if (b.n >= bytes) return SCARL_OK;
   const size_t want = bytes;
+  if (ctx->used - b.n + want > ctx->budget) drop_dct_tabs(ctx);
   if (ctx->used - b.n + want > ctx->budget)
     return fail(ctx, SCARL_ENOMEM, "device memory budget exceeded (" + std::to_string(want) + " bytes requested)");
-  if (b.p) {
-    cudaFree(b.p);
-    ctx->used -= b.n;
-    b.p = nullptr;
-    b.n = 0;
-  }
+  release(ctx, b);
   cudaError_t e = cudaMalloc(&b.p, want);
+  if (e != cudaSuccess && drop_dct_tabs(ctx)) {
+    cudaGetLastError();
+    e = cudaMalloc(&b.p, want);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     b.p = nullptr;
@@ -236,15 +270,6 @@ int ensure(scarl_ctx* ctx, Buf& b, size_t bytes) {
   b.n = want;
   ctx->used += want;
   return SCARL_OK;
-}
-
-void release(scarl_ctx* ctx, Buf& b) {
-  if (b.p) {
-    cudaFree(b.p);
-    ctx->used -= b.n;
-  }
-  b.p = nullptr;
-  b.n = 0;
 }
 
 bool is_device_ptr(const void* p) {
@@ -1307,30 +1332,51 @@ int upload_blend_tables(scarl_ctx* ctx, const scarl_layout& lay, int partitionTy
   return SCARL_OK;
 }
 
-// Folded cosine matrix of a DCT-III of length N over K inputs, kept by the context.
-int dct_table(scarl_ctx* ctx, int N, int K, const double** out) {
-  const std::pair<int, int> key(N, K);
-  auto it = ctx->dct_tabs.find(key);
-  if (it != ctx->dct_tabs.end()) {
-    *out = (const double*)it->second.p;
-    return SCARL_OK;
+// The cosines of a DCT-III of length N over K inputs: the folded matrix (*tab),
+// or, where it would exceed kDctTab or finds no room, the 4 N roots that the
+// kernel forms it from (*roots).  Kept by the context, kDctTabs bytes in all
+// beside what the call in progress uses (dct_held).
+int dct_table(scarl_ctx* ctx, int N, int K, const double** tab, const double** roots) {
+  *tab = *roots = nullptr;
+  const size_t mat = (size_t)K * round_up((N + 1) / 2, 2) * 8, raw = (size_t)4 * N * 8;
+  auto find = [&](int k) -> const double* {
+    const std::pair<int, int> key(N, k);
+    const auto it = ctx->dct_tabs.find(key);
+    if (it == ctx->dct_tabs.end()) return nullptr;
+    ctx->dct_held.push_back(key);
+    return (const double*)it->second.p;
+  };
+  if ((*tab = find(K)) || (mat > kDctTab && (*roots = find(0)))) return SCARL_OK;
+  size_t kept = 0;
+  for (const auto& t : ctx->dct_tabs) kept += t.second.n;
+  if (kept + std::max(raw, mat <= kDctTab ? mat : 0) > kDctTabs) drop_dct_tabs(ctx);
+  Buf r, b;
+  *roots = find(0);
+  if (!*roots) {
+    RC(ensure(ctx, r, raw));
+    std::vector<double> c(4 * (size_t)N);
+    for (int64_t m = 0; m < 4 * (int64_t)N; ++m) c[m] = std::cos(M_PI * (double)m / (2.0 * (double)N));
+    if (cudaMemcpy(r.p, c.data(), raw, cudaMemcpyHostToDevice) != cudaSuccess) {
+      release(ctx, r);
+      return fail(ctx, SCARL_EDEVICE, std::string("cosine table: ") + cudaGetErrorString(cudaGetLastError()));
+    }
+    *roots = (const double*)r.p;
   }
-  Buf raw, b;
-  RC(ensure(ctx, raw, (size_t)4 * N * 8));
-  std::vector<double> c(4 * (size_t)N);
-  for (int m = 0; m < 4 * N; ++m) c[m] = std::cos(M_PI * (double)m / (2.0 * (double)N));
-  int rc = ensure(ctx, b, (size_t)K * round_up((N + 1) / 2, 2) * 8);
-  if (rc == SCARL_OK && (cudaMemcpy(raw.p, c.data(), c.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
-                         launch_dct_table((const double*)raw.p, N, K, (double*)b.p, ctx->stream) != cudaSuccess ||
-                         cudaStreamSynchronize(ctx->stream) != cudaSuccess))
-    rc = fail(ctx, SCARL_EDEVICE, std::string("cosine table: ") + cudaGetErrorString(cudaGetLastError()));
-  release(ctx, raw);
-  if (rc != SCARL_OK) {
-    release(ctx, b);
-    return rc;
+  if (mat <= kDctTab && ensure(ctx, b, mat) == SCARL_OK) {
+    const bool ok = launch_dct_table(*roots, N, K, (double*)b.p, ctx->stream) == cudaSuccess &&
+                    cudaStreamSynchronize(ctx->stream) == cudaSuccess;
+    release(ctx, r);
+    if (!ok) {
+      release(ctx, b);
+      return fail(ctx, SCARL_EDEVICE, std::string("cosine table: ") + cudaGetErrorString(cudaGetLastError()));
+    }
+    ctx->dct_tabs[{N, K}] = b;
+    *roots = nullptr;
+    *tab = find(K);
+  } else if (r.p) {
+    ctx->dct_tabs[{N, 0}] = r;
+    find(0);
   }
-  ctx->dct_tabs[key] = b;
-  *out = (const double*)b.p;
   return SCARL_OK;
 }
 
@@ -1350,13 +1396,18 @@ int dct_tiles(scarl_ctx* ctx, int nt, const int Np[3], const double* xRange, con
     a.corrL[d] = corrL[d];
     nexp += (size_t)a.K[d];
   }
-  for (int d = 0; d < 3; ++d) RC(dct_table(ctx, Np[d], a.K[d], &a.tab[d]));
   int64_t nsk, n1, n2;
   dct_sizes(a.Np, a.K, &nsk, &n1, &n2);
   RC(ensure(ctx, ctx->sk, (size_t)nsk * nt * 8));
   RC(ensure(ctx, ctx->t1, (size_t)n1 * nt * 8));
   RC(ensure(ctx, ctx->t2, (size_t)n2 * nt * 8));
   RC(ensure(ctx, ctx->dtabs, nexp * nt * 8));
+  // the tables last: what they can do without must not keep the buffers out
+  struct Hold {
+    scarl_ctx* c;
+    ~Hold() { c->dct_held.clear(); }
+  } hold{ctx};
+  for (int d = 0; d < 3; ++d) RC(dct_table(ctx, Np[d], a.K[d], &a.tab[d], &a.roots[d]));
   // per-axis exp(-PI k^2) factors, SRC_F/fftw_ScaRL.f90:300-326
   void* hp;
   RC(pinned(ctx, nexp * nt * 8, &hp));

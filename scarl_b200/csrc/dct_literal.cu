@@ -80,6 +80,18 @@ __global__ void k_dct_table(const double* __restrict__ ctab, int N, int K, int H
   }
 }
 
+// The same value formed in the kernel, for axes whose matrix would be too large
+// to keep: x mod 4 N by Barrett's reduction, inv = floor((2^64 - 1) / 4 N) (the
+// quotient comes out right or one short).
+__device__ __forceinline__ double dct_cosine(const double* __restrict__ ctab, int N, uint64_t inv, int i, int c) {
+  if (c >= (N + 1) / 2) return 0.0;
+  if (i == 0) return 1.0;
+  const uint64_t d = 4 * (uint64_t)N, x = (uint64_t)i * (uint64_t)(2 * (int64_t)c + 1);
+  uint64_t m = x - __umul64hi(x, inv) * d;
+  if (m >= d) m -= d;
+  return 2.0 * __ldg(ctab + m);
+}
+
 cudaError_t launch_dct_table(const double* ctab, int N, int K, double* tab, cudaStream_t s) {
   const int H = (N + 1) / 2, hp = (H + 1) / 2 * 2;
   const int64_t n = (int64_t)K * hp;
@@ -92,6 +104,8 @@ struct DctMM {
   const double* A;
   const double* B;
   double* D;
+  const double* ctab;     // cos(pi m / (2 Nfull)) where the cosine operand is formed from it, else null
+  uint64_t inv;           // of 4 Nfull (dct_cosine)
   int64_t lda, ldb, ldd;  // row strides (elements, even for A and B)
   int64_t bA, bB, bD;
   int wa, wb;             // readable elements of a row of A and B (even)
@@ -130,9 +144,12 @@ enum MmOut { MM_FOLD_N, MM_FOLD_M, MM_FINAL, MM_FINAL_EXP };
 // next tile's first copies in flight during the current tile's output.  Warps:
 // 2 along m (interleaved groups of 16 rows, so that a partial last tile keeps
 // both busy) x 4 along n.
-template <int MW, int OUT>
+// ROOTS: the cosine operand (B in the x step, A in the others) is formed from
+// p.ctab instead of copied.
+template <int MW, int OUT, bool ROOTS>
 __global__ void __launch_bounds__(256, 2) k_dct_mm(const DctMM p) {
   using Cfg = MmCfg<MW>;
+  constexpr bool COS_A = ROOTS && OUT != MM_FOLD_N, COS_B = ROOTS && OUT == MM_FOLD_N;
   constexpr bool EXP = OUT == MM_FINAL_EXP;
   extern __shared__ __align__(16) double mm_sm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -153,24 +170,44 @@ __global__ void __launch_bounds__(256, 2) k_dct_mm(const DctMM p) {
   const unsigned db = sm0 + 8 * (2 * kMmKB * Cfg::SA + slot_row(rb, Cfg::SB) + qb);
   const double *pa = nullptr, *pb = nullptr;
   int ka = 0, kb_ = 0;
+  int m0n = 0, n0n = 0;
+  unsigned btn = 0;
   auto load = [&](int kb, int slot) {
     const int i0 = 2 * kMmKB * kb;
     const unsigned so = slot * (Cfg::STAGE * 8);
 #pragma unroll
     for (int u = 0; u < UA; ++u) {
+      if constexpr (COS_A) continue;
       const bool ok = i0 + RA * u < ka;
       cp16_zfill(da + so + 8 * (RA / 2) * Cfg::SA * u, ok ? pa + (int64_t)(RA * u) * p.lda : p.A, ok ? 16 : 0);
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
+      if constexpr (COS_B) continue;
       const bool ok = i0 + 8 * u < kb_;
       cp16_zfill(db + so + 8 * 4 * Cfg::SB * u, ok ? pb + (int64_t)(8 * u) * p.ldb : p.B, ok ? 16 : 0);
     }
     pa += 2 * kMmKB * p.lda;
     pb += 2 * kMmKB * p.ldb;
   };
-  int m0n = 0, n0n = 0;
-  unsigned btn = 0;
+  // ROOTS: the thread's cosines of a stage, in registers until the current stage
+  // has been multiplied
+  constexpr int UC = !ROOTS ? 1 : COS_A ? UA : 2;
+  double2 cosv[UC];
+  auto form = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < (ROOTS ? UC : 0); ++u) {
+      const int i = 2 * kMmKB * kb + (COS_A ? ra + RA * u : rb + 8 * u), c = COS_A ? m0n + qa : n0n + qb;
+      cosv[u] = i < p.K ? make_double2(dct_cosine(p.ctab, p.Nfull, p.inv, i, c), dct_cosine(p.ctab, p.Nfull, p.inv, i, c + 1))
+                        : make_double2(0.0, 0.0);
+    }
+  };
+  auto put = [&](int slot) {
+    double* st = mm_sm + slot * Cfg::STAGE + (COS_A ? slot_row(ra, Cfg::SA) + qa : 2 * kMmKB * Cfg::SA + slot_row(rb, Cfg::SB) + qb);
+#pragma unroll
+    for (int u = 0; u < (ROOTS ? UC : 0); ++u)
+      *reinterpret_cast<double2*>(st + (COS_A ? (RA / 2) * Cfg::SA : 4 * Cfg::SB) * u) = cosv[u];
+  };
   auto start = [&](unsigned tile) {  // the tile's coordinates and first copies
     const unsigned rest = tile / p.nm;
     m0n = (int)(tile - rest * p.nm) * Cfg::MT;
@@ -182,7 +219,11 @@ __global__ void __launch_bounds__(256, 2) k_dct_mm(const DctMM p) {
     kb_ = n0n + qb < p.wb ? p.K - rb : 0;
 #pragma unroll
     for (int s = 0; s < kMmStages - 1; ++s) {
-      if (s < nk) load(s, s);
+      if (s < nk) {
+        load(s, s);
+        form(s);
+        put(s);
+      }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
   };
@@ -209,7 +250,11 @@ __global__ void __launch_bounds__(256, 2) k_dct_mm(const DctMM p) {
       for (int kb = 0; kb < nk; ++kb) {
         asm volatile("cp.async.wait_group %0;\n" ::"n"(kMmStages - 2) : "memory");
         __syncthreads();
-        if (kb + kMmStages - 1 < nk) load(kb + kMmStages - 1, (kb + kMmStages - 1) % kMmStages);
+        const bool more = kb + kMmStages - 1 < nk;
+        if (more) {
+          load(kb + kMmStages - 1, (kb + kMmStages - 1) % kMmStages);
+          form(kb + kMmStages - 1);
+        }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         if constexpr (GW > 0) {
           const double* as = mm_sm + (kb % kMmStages) * Cfg::STAGE;
@@ -227,6 +272,7 @@ __global__ void __launch_bounds__(256, 2) k_dct_mm(const DctMM p) {
             }
           }
         }
+        if (more) put((kb + kMmStages - 1) % kMmStages);
       }
     };
     if (mw == 0) loop(std::integral_constant<int, 0>());
@@ -335,22 +381,26 @@ __global__ void __launch_bounds__(256, 2) k_dct_mm(const DctMM p) {
   }
 }
 
-template <int MW, int OUT> static cudaError_t run_mm_w(DctMM p, int64_t batch, cudaStream_t s) {
+template <int MW, int OUT, bool ROOTS> static cudaError_t run_mm_w(DctMM p, int64_t batch, cudaStream_t s) {
   using Cfg = MmCfg<MW>;
   p.nm = (p.M + Cfg::MT - 1) / Cfg::MT;
   p.nn = (p.N + kMmNT - 1) / kMmNT;
   const int64_t tiles = (int64_t)p.nm * p.nn * batch;
   if (tiles < 1 || tiles > 2147483647LL) return cudaErrorInvalidValue;
   p.batch = (int)batch;
-  const cudaError_t e = cudaFuncSetAttribute(k_dct_mm<MW, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+  p.inv = ~(uint64_t)0 / (4 * (uint64_t)p.Nfull);
+  const cudaError_t e = cudaFuncSetAttribute(k_dct_mm<MW, OUT, ROOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
   if (e != cudaSuccess) return e;
-  k_dct_mm<MW, OUT><<<(unsigned)std::min<int64_t>(tiles, 2 * 148), 256, Cfg::SMEM, s>>>(p);
+  k_dct_mm<MW, OUT, ROOTS><<<(unsigned)std::min<int64_t>(tiles, 2 * 148), 256, Cfg::SMEM, s>>>(p);
   return cudaGetLastError();
 }
-// Tiles of 64 rows reuse a B fragment most; 32 and 16 only where M is that small.
+// Tiles of 64 rows reuse a B fragment most; 32 only where M is that small.
+template <int OUT, bool ROOTS> static cudaError_t run_mm_r(const DctMM& p, int64_t batch, cudaStream_t s) {
+  if (p.M <= 32) return run_mm_w<2, OUT, ROOTS>(p, batch, s);
+  return run_mm_w<4, OUT, ROOTS>(p, batch, s);
+}
 template <int OUT> static cudaError_t run_mm(const DctMM& p, int64_t batch, cudaStream_t s) {
-  if (p.M <= 32) return run_mm_w<2, OUT>(p, batch, s);
-  return run_mm_w<4, OUT>(p, batch, s);
+  return p.ctab ? run_mm_r<OUT, true>(p, batch, s) : run_mm_r<OUT, false>(p, batch, s);
 }
 
 void dct_sizes(const int Np[3], const int K[3], int64_t* sk, int64_t* t1, int64_t* t2) {
@@ -376,17 +426,20 @@ cudaError_t launch_dct_literal(const DctArgs& a_in, cudaStream_t s) {
   DctMM p{};
   // x: rows (j, k) of the octant
   p.A = a.sk; p.lda = a.lp; p.wa = (int)a.lp; p.bA = nsk;
+  p.ctab = a.roots[0];
   p.B = a.tab[0]; p.ldb = hp[0]; p.wb = hp[0]; p.bB = 0;
   p.D = a.t1; p.ldd = n0p; p.bD = n1;
   p.M = K1 * K2; p.N = H[0]; p.K = K0; p.Nfull = N0;
   if ((e = run_mm<MM_FOLD_N>(p, a.nt, s)) != cudaSuccess) return e;
   // y: per kz (and tile), rows of x
+  p.ctab = a.roots[1];
   p.A = a.tab[1]; p.lda = hp[1]; p.wa = hp[1]; p.bA = 0;
   p.B = a.t1; p.ldb = n0p; p.wb = n0p; p.bB = (int64_t)K1 * n0p;
   p.D = a.t2; p.ldd = n0p; p.bD = (int64_t)N1 * n0p;
   p.M = H[1]; p.N = n0p; p.K = K1; p.Nfull = N1;
   if ((e = run_mm<MM_FOLD_M>(p, (int64_t)K2 * a.nt, s)) != cudaSuccess) return e;
   // z: whole planes, through the output stage
+  p.ctab = a.roots[2];
   p.A = a.tab[2]; p.lda = hp[2]; p.wa = hp[2]; p.bA = 0;
   p.B = a.t2; p.ldb = N1 * n0p; p.wb = N1 * n0p; p.bB = n2;
   p.D = nullptr; p.ldd = 0; p.bD = (int64_t)N0 * N1 * N2;

@@ -161,7 +161,8 @@ struct DctArgs {
   double* sk;           // spectra, dct_sizes elements a tile
   double* t1;           // after the x transform
   double* t2;           // after the y transform
-  const double* tab[3];  // folded cosines of each axis (launch_dct_table)
+  const double* tab[3];  // folded cosines of each axis (launch_dct_table), or null and
+  const double* roots[3];  // cos(pi m / (2 N)), m < 4N, from which they are formed
   Epilogue epi;         // output stage; nt > 1: plain tiles one after the other at epi.out
 };
 cudaError_t launch_dct_literal(const DctArgs& a, cudaStream_t s);
