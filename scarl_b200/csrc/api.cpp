@@ -272,6 +272,16 @@ int ensure(scarl_ctx* ctx, Buf& b, size_t bytes) {
   return SCARL_OK;
 }
 
+// Host table -> device on the context's stream, complete on return.  (A plain
+// cudaMemcpy returns once pageable memory is staged, and the stream, created
+// non-blocking, does not wait for the legacy one: a kernel launched next could read
+// the table before it arrives.)
+int put_table(scarl_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return SCARL_OK;
+}
+
 bool is_device_ptr(const void* p) {
   if (!p) return false;
   cudaPointerAttributes a;
@@ -399,7 +409,7 @@ int check_status(scarl_ctx* ctx) {
   int st = 0;
   CK(cudaMemcpy(&st, ctx->status.p, sizeof st, cudaMemcpyDeviceToHost));
   if (st == 0) return SCARL_OK;
-  CK(cudaMemset(ctx->status.p, 0, sizeof st));
+  CK(cudaMemsetAsync(ctx->status.p, 0, sizeof st, ctx->stream));
   return fail(ctx, SCARL_ETIMEOUT, "a bounded tensor-core or copy wait expired; the output is invalid");
 }
 
@@ -613,7 +623,7 @@ int slab_end(SlabCopier& c) {
 int ensure_status(scarl_ctx* ctx) {
   if (!ctx->status.p) {
     RC(ensure(ctx, ctx->status, 16));
-    CK(cudaMemset(ctx->status.p, 0, 16));
+    CK(cudaMemsetAsync(ctx->status.p, 0, 16, ctx->stream));
   }
   return SCARL_OK;
 }
@@ -671,10 +681,10 @@ int twiddles(scarl_ctx* ctx, int P, int dt, const void** out) {
     d[2 * m + 1] = (double)sinl(a);
   }
   if (dt == 8) {
-    CK(cudaMemcpy(b.p, d.data(), d.size() * 8, cudaMemcpyHostToDevice));
+    RC(put_table(ctx, b.p, d.data(), d.size() * 8));
   } else {
     std::vector<float> f(d.begin(), d.end());
-    CK(cudaMemcpy(b.p, f.data(), f.size() * 4, cudaMemcpyHostToDevice));
+    RC(put_table(ctx, b.p, f.data(), f.size() * 4));
   }
   ctx->twiddles[key] = b;
   *out = b.p;
@@ -744,7 +754,7 @@ int padded_plan(scarl_ctx* ctx, int dt, const int P[3], const double dx[3],
     h.insert(h.end(), r[0].begin(), r[0].end());
     h.insert(h.end(), r[1].begin(), r[1].end());
     h.insert(h.end(), r[2].begin(), r[2].end());
-    CK(cudaMemcpy(t64.p, h.data(), tot * 8, cudaMemcpyHostToDevice));
+    RC(put_table(ctx, t64.p, h.data(), tot * 8));
     const double* d0 = (const double*)t64.p;
     const double* d1 = d0 + n[0];
     const double* d2 = d1 + n[1];
@@ -794,10 +804,10 @@ int padded_plan(scarl_ctx* ctx, int dt, const int P[3], const double dx[3],
   }
   RC(ensure(ctx, pl.tabs, tab.size() * dt));
   if (dt == 8) {
-    CK(cudaMemcpy(pl.tabs.p, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice));
+    RC(put_table(ctx, pl.tabs.p, tab.data(), tab.size() * 8));
   } else {
     std::vector<float> f(tab.begin(), tab.end());
-    CK(cudaMemcpy(pl.tabs.p, f.data(), f.size() * 4, cudaMemcpyHostToDevice));
+    RC(put_table(ctx, pl.tabs.p, f.data(), f.size() * 4));
   }
   for (int s = 0; s < 6; ++s) pl.t[s] = (const char*)pl.tabs.p + off[s] * dt;
   if (pl.amp == AMP_SEPARABLE) pl.t[3] = pl.t[4] = pl.t[5] = nullptr;
@@ -816,7 +826,7 @@ int pm_powers(scarl_ctx* ctx, const uint32_t** out) {
       h[i] = (uint32_t)b;
       b = (b * b) % 2147483647ull;
     }
-    CK(cudaMemcpy(ctx->pmpw.p, h, sizeof h, cudaMemcpyHostToDevice));
+    RC(put_table(ctx, ctx->pmpw.p, h, sizeof h));
   }
   *out = (const uint32_t*)ctx->pmpw.p;
   return SCARL_OK;
@@ -1089,7 +1099,7 @@ int ens_maps(scarl_ctx* ctx, EnsPlan* e) {
     h.insert(h.end(), g.start.begin(), g.start.end());
   }
   RC(ensure(ctx, e->dmap, h.size() * sizeof(int)));
-  CK(cudaMemcpy(e->dmap.p, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
+  RC(put_table(ctx, e->dmap.p, h.data(), h.size() * sizeof(int)));
   ctx->h2d += h.size() * sizeof(int);
   const int* base = static_cast<const int*>(e->dmap.p);
   for (size_t k = 0; k < e->groups.size(); ++k) {
@@ -1239,7 +1249,7 @@ int ens_tune(scarl_ctx* ctx, EnsPlan* e) {
       if (ens_starts(ctx, e, g, v, &st) != SCARL_OK) continue;
       CK(cudaStreamSynchronize(ctx->stream));
       RC(ensure(ctx, e->tmp, st.size() * sizeof(int)));
-      CK(cudaMemcpy(e->tmp.p, st.data(), st.size() * sizeof(int), cudaMemcpyHostToDevice));
+      RC(put_table(ctx, e->tmp.p, st.data(), st.size() * sizeof(int)));
       BatchMap m = g.m;
       m.start = static_cast<const int*>(e->tmp.p);
       m.total = st.back();
@@ -1356,9 +1366,10 @@ int dct_table(scarl_ctx* ctx, int N, int K, const double** tab, const double** r
     RC(ensure(ctx, r, raw));
     std::vector<double> c(4 * (size_t)N);
     for (int64_t m = 0; m < 4 * (int64_t)N; ++m) c[m] = std::cos(M_PI * (double)m / (2.0 * (double)N));
-    if (cudaMemcpy(r.p, c.data(), raw, cudaMemcpyHostToDevice) != cudaSuccess) {
+    const int rc = put_table(ctx, r.p, c.data(), raw);
+    if (rc != SCARL_OK) {
       release(ctx, r);
-      return fail(ctx, SCARL_EDEVICE, std::string("cosine table: ") + cudaGetErrorString(cudaGetLastError()));
+      return rc;
     }
     *roots = (const double*)r.p;
   }
@@ -2149,10 +2160,10 @@ int scarl_mlp_init(scarl_ctx* ctx, uint64_t seed) {
   for (int i = 0; i < H * H; ++i) p[o++] = (float)(normal() * std::sqrt(2.0 / H));
   o += H;
   for (int i = 0; i < O * H; ++i) p[o++] = (float)(normal() * std::sqrt(1.0 / H));
-  CK(cudaMemcpy(ctx->mlp_p.p, p.data(), (size_t)kMlpParams * 4, cudaMemcpyHostToDevice));
-  CK(cudaMemset(ctx->mlp_m.p, 0, (size_t)kMlpParams * 4));
-  CK(cudaMemset(ctx->mlp_v.p, 0, (size_t)kMlpParams * 4));
-  CK(cudaMemset(ctx->mlp_g.p, 0, (size_t)kMlpParams * 4));
+  RC(put_table(ctx, ctx->mlp_p.p, p.data(), (size_t)kMlpParams * 4));
+  CK(cudaMemsetAsync(ctx->mlp_m.p, 0, (size_t)kMlpParams * 4, ctx->stream));
+  CK(cudaMemsetAsync(ctx->mlp_v.p, 0, (size_t)kMlpParams * 4, ctx->stream));
+  CK(cudaMemsetAsync(ctx->mlp_g.p, 0, (size_t)kMlpParams * 4, ctx->stream));
   CK(launch_to_bf16((const float*)ctx->mlp_p.p, ctx->mlp_wb.p, kMlpParams, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->h2d += (size_t)kMlpParams * 4;
@@ -2165,10 +2176,10 @@ int scarl_mlp_params(scarl_ctx* ctx, float* get, const float* set) {
   RC(begin(ctx));
   if (set) {
     RC(mlp_alloc(ctx));
-    CK(cudaMemcpy(ctx->mlp_p.p, set, (size_t)kMlpParams * 4, cudaMemcpyHostToDevice));
-    CK(cudaMemset(ctx->mlp_m.p, 0, (size_t)kMlpParams * 4));
-    CK(cudaMemset(ctx->mlp_v.p, 0, (size_t)kMlpParams * 4));
-    CK(cudaMemset(ctx->mlp_g.p, 0, (size_t)kMlpParams * 4));
+    RC(put_table(ctx, ctx->mlp_p.p, set, (size_t)kMlpParams * 4));
+    CK(cudaMemsetAsync(ctx->mlp_m.p, 0, (size_t)kMlpParams * 4, ctx->stream));
+    CK(cudaMemsetAsync(ctx->mlp_v.p, 0, (size_t)kMlpParams * 4, ctx->stream));
+    CK(cudaMemsetAsync(ctx->mlp_g.p, 0, (size_t)kMlpParams * 4, ctx->stream));
     CK(launch_to_bf16((const float*)ctx->mlp_p.p, ctx->mlp_wb.p, kMlpParams, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->mlp_ready = true;
@@ -2176,7 +2187,8 @@ int scarl_mlp_params(scarl_ctx* ctx, float* get, const float* set) {
   }
   if (get) {
     if (!ctx->mlp_ready) return fail(ctx, SCARL_EINVAL, "no model: call scarl_mlp_init or set parameters");
-    CK(cudaMemcpy(get, ctx->mlp_p.p, (size_t)kMlpParams * 4, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(get, ctx->mlp_p.p, (size_t)kMlpParams * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
   }
   return SCARL_OK;
 }
