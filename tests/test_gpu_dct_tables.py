@@ -73,6 +73,11 @@ def test_long_axis_small_budget():
         check(c, (40001, 3, 4))
 
 
+@pytest.mark.parametrize("Np", [(131073, 2, 3), (131072, 3, 2), (140001, 4, 2)])
+def test_more_inputs_than_a_grid_dimension(ctx, Np):
+    check(ctx, Np)
+
+
 def test_many_lengths_one_context():
     """Matrices of 40 lengths (over 20 MB together) pass through a context of 8 MB,
     and leave room for another generator's 5 MB; those of long axes (67 MB each)
