@@ -2859,24 +2859,36 @@ int scarl_generate_sample(scarl_ctx* ctx, const scarl_sample* s, const scarl_gen
     for (int d = 0; d < 3; ++d)
       if (lay.Np[d] < 2) return fail(ctx, SCARL_EINVAL, "Np must be >= 2");
   }
-  // literal tiles that fit kDctBatch bytes together, and the budget with their
-  // work buffers: one launch per step over all of them, then one gather of the
-  // blended field; larger ones one after the other, each blended by its z
-  // transform's output stage
-  bool dct_batch = gen == SCARL_GEN_DCT && lay.nb_tiles > 1 && ntile * 8 * lay.nb_tiles <= kDctBatch;
-  if (dct_batch) {
-    const int K[3] = {lay.Np[0] / 2, lay.Np[1] / 2, lay.Np[2] / 2};
-    int64_t nsk, n1, n2;
-    dct_sizes(lay.Np, K, &nsk, &n1, &n2);
-    const Buf* bufs[4] = {&ctx->tile, &ctx->sk, &ctx->t1, &ctx->t2};
-    const size_t want[4] = {ntile * 8, (size_t)nsk * 8, (size_t)n1 * 8, (size_t)n2 * 8};
-    size_t more = (size_t)1 << 20;  // the axes' tables
-    for (int i = 0; i < 4; ++i) more += want[i] * lay.nb_tiles > bufs[i]->n ? want[i] * lay.nb_tiles - bufs[i]->n : 0;
-    dct_batch = ctx->used + more <= ctx->budget && ensure(ctx, ctx->tile, ntile * 8 * lay.nb_tiles) == SCARL_OK;
-  }
   const void* phi_all = nullptr;
   if (gen == SCARL_GEN_DCT && o.phiK)
     RC(in_dev(ctx, ctx->stage_in, o.phiK, nk * lay.nb_tiles * 8, &phi_all));
+  // literal tiles that fit kDctBatch bytes together: one launch per step over all
+  // of them, then one gather of the blended field.  Larger ones, and those whose
+  // buffers together find no room, one after the other, each blended by its z
+  // transform's output stage.
+  bool dct_batch = gen == SCARL_GEN_DCT && lay.nb_tiles > 1 && ntile * 8 * lay.nb_tiles <= kDctBatch;
+  if (dct_batch) {
+    std::vector<double> xr((size_t)3 * lay.nb_tiles);
+    for (int q = 0; q < lay.nb_tiles; ++q) {
+      scarl_tile tq;
+      tile_geometry(&lay, s->xMinGlob, q, &tq);
+      std::memcpy(&xr[3 * (size_t)q], tq.xRange, sizeof tq.xRange);
+    }
+    int rc = ensure(ctx, ctx->tile, ntile * 8 * lay.nb_tiles);
+    if (rc == SCARL_OK) {
+      Epilogue plain;
+      std::memset(&plain, 0, sizeof plain);
+      plain.out = ctx->tile.p;
+      rc = dct_tiles(ctx, lay.nb_tiles, lay.Np, xr.data(), s->corrL, (const double*)phi_all, nullptr,
+                     (uint32_t)s->seedBase + 1u, false, plain);
+    }
+    if (rc == SCARL_ENOMEM) {  // before any launch: give the batch's buffers back
+      dct_batch = false;
+      for (Buf* b : {&ctx->tile, &ctx->sk, &ctx->t1, &ctx->t2, &ctx->dtabs}) release(ctx, *b);
+    } else if (rc != SCARL_OK) {
+      return rc;
+    }
+  }
   // pinned host output over several rows of tiles: finished boxes stream
   // back while the later rows are generated
   SlabCopier slabs;
@@ -2999,16 +3011,6 @@ int scarl_generate_sample(scarl_ctx* ctx, const scarl_sample* s, const scarl_gen
         if (!dct_batch) {
           RC(dct_tiles(ctx, 1, lay.Np, t.xRange, s->corrL, phi, nullptr, (uint32_t)seedStart, gm == SCARL_FFT_MPI, e));
         } else if (r == 0) {
-          std::vector<double> xr((size_t)3 * lay.nb_tiles);
-          for (int q = 0; q < lay.nb_tiles; ++q) {
-            scarl_tile tq;
-            tile_geometry(&lay, s->xMinGlob, q, &tq);
-            std::memcpy(&xr[3 * (size_t)q], tq.xRange, sizeof tq.xRange);
-          }
-          Epilogue plain;
-          std::memset(&plain, 0, sizeof plain);
-          plain.out = ctx->tile.p;
-          RC(dct_tiles(ctx, lay.nb_tiles, lay.Np, xr.data(), s->corrL, phi, nullptr, (uint32_t)seedStart, false, plain));
           BlendGather g;
           std::memset(&g, 0, sizeof g);
           g.tiles = (const double*)ctx->tile.p;
