@@ -42,34 +42,34 @@ namespace scarl {
 
 constexpr double kPiRefD = 3.1415926535898;  // SRC_F/constants_ScaRL.f90:5
 
-// One thread per mode: blocks of 128 consecutive lines l = j + K1 k of one (i,
-// tile), all of them along gridDim.x (2^31 - 1 blocks, where y and z end at
-// 65535: an axis may have more inputs than that).
-__global__ void __launch_bounds__(128) k_dct_spec(const DctArgs a, int lblocks) {
-  const unsigned it = blockIdx.x / (unsigned)lblocks;
-  const int nl = a.K[1] * a.K[2], l = (int)((blockIdx.x - it * lblocks) * 128 + threadIdx.x);
+// One thread per mode: blockIdx.x * 128 + threadIdx.x is the line l = j + K1 k,
+// blockIdx.z the tile, i walks from blockIdx.y by gridDim.y (at most 65535; an
+// axis may have more inputs).
+__global__ void __launch_bounds__(128) k_dct_spec(const DctArgs a) {
+  const int nl = a.K[1] * a.K[2], l = (int)(blockIdx.x * 128 + threadIdx.x);
   if (l >= nl) return;
-  const int tile = (int)(it / (unsigned)a.K[0]), i = (int)(it - (unsigned)tile * a.K[0]);
-  const int k = l / a.K[1], j = l - k * a.K[1];
-  const double* cx = a.cexp + (int64_t)tile * (a.K[0] + a.K[1] + a.K[2]);
-  const double* cy = cx + a.K[0];
-  const double* cz = cy + a.K[1];
-  const int64_t o = i + (int64_t)a.K[0] * l, n = (int64_t)a.K[0] * nl;  // the reference's element order
-  double S = 1.0;
-  S = __dmul_rn(__dmul_rn(S, a.corrL[0]), cx[i]);
-  S = __dmul_rn(__dmul_rn(S, a.corrL[1]), cy[j]);
-  S = __dmul_rn(__dmul_rn(S, a.corrL[2]), cz[k]);
-  double phi;
-  if (a.phi) {
-    phi = a.phi[tile * n + o];
-  } else {
-    const u32x4 q = philox4x32_10({(uint32_t)o, (uint32_t)((uint64_t)o >> 32), a.stream, 1u},
-                                  a.k0 + (uint32_t)tile, a.k1);
-    phi = u01_d(q.x, q.y);
+  const int tile = blockIdx.z, k = l / a.K[1], j = l - k * a.K[1];
+  for (int i = blockIdx.y; i < a.K[0]; i += gridDim.y) {
+    const double* cx = a.cexp + (int64_t)tile * (a.K[0] + a.K[1] + a.K[2]);
+    const double* cy = cx + a.K[0];
+    const double* cz = cy + a.K[1];
+    const int64_t o = i + (int64_t)a.K[0] * l, n = (int64_t)a.K[0] * nl;  // the reference's element order
+    double S = 1.0;
+    S = __dmul_rn(__dmul_rn(S, a.corrL[0]), cx[i]);
+    S = __dmul_rn(__dmul_rn(S, a.corrL[1]), cy[j]);
+    S = __dmul_rn(__dmul_rn(S, a.corrL[2]), cz[k]);
+    double phi;
+    if (a.phi) {
+      phi = a.phi[tile * n + o];
+    } else {
+      const u32x4 q = philox4x32_10({(uint32_t)o, (uint32_t)((uint64_t)o >> 32), a.stream, 1u},
+                                    a.k0 + (uint32_t)tile, a.k1);
+      phi = u01_d(q.x, q.y);
+    }
+    const double g = a.gamma ? a.gamma[tile * n + o] : 1.0;
+    const double c = cos(__dmul_rn(__dmul_rn(2.0, kPiRefD), phi));
+    a.sk[((int64_t)tile * a.K[0] + i) * a.lp + l] = __dmul_rn(__dmul_rn(g, sqrt(S)), c);
   }
-  const double g = a.gamma ? a.gamma[tile * n + o] : 1.0;
-  const double c = cos(__dmul_rn(__dmul_rn(2.0, kPiRefD), phi));
-  a.sk[((int64_t)tile * a.K[0] + i) * a.lp + l] = __dmul_rn(__dmul_rn(g, sqrt(S)), c);
 }
 
 // tab[i][n] = c_i cos(pi i (2n + 1) / (2N)), i < K, n < H = (N + 1) / 2, rows
@@ -423,10 +423,7 @@ cudaError_t launch_dct_literal(const DctArgs& a_in, cudaStream_t s) {
   dct_sizes(a.Np, a.K, &nsk, &n1, &n2);
   if ((int64_t)N1 * n0p > 2147483647LL - 64 || (int64_t)K1 * K2 > 2147483647LL - 64) return cudaErrorInvalidValue;
   a.lp = ((int64_t)K1 * K2 + 1) / 2 * 2;
-  const int lblocks = (K1 * K2 + 127) / 128;
-  const int64_t blocks = (int64_t)lblocks * K0 * a.nt;
-  if (blocks > 2147483647LL) return cudaErrorInvalidValue;  // over 1 TB of spectrum
-  k_dct_spec<<<(unsigned)blocks, 128, 0, s>>>(a, lblocks);
+  k_dct_spec<<<dim3((unsigned)((K1 * K2 + 127) / 128), std::min(K0, 65535), a.nt), 128, 0, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   DctMM p{};
