@@ -3396,6 +3396,11 @@ int scarl_rebuild_sk(scarl_ctx* ctx, const void* field, int dtype, const int L[3
       }
     }
   }
+  // (x - avg) / stdDev is squared at a magnitude about 1 as in the reference: the
+  // window carries stdDev's power of two (exact), what is left of it divides the sums
+  const int ex = std::max(-1000, std::min(1000, std::isinf(stdDev) ? 0 : std::ilogb(stdDev)));
+  const double scale = std::ldexp(1.0, -ex), sd = stdDev * scale;
+  for (size_t i = 0; i < nw; ++i) ((double*)hp)[i] *= scale;
   RC(upload_pinned(ctx, ctx->tabs.p, nw * 8));
   size_t o = 0;
   for (int d = 0; d < 3; o += L[d], ++d) {
@@ -3412,7 +3417,7 @@ int scarl_rebuild_sk(scarl_ctx* ctx, const void* field, int dtype, const int L[3
     const int nl = L[d], nkeep = nl / 2;
     // linear lag sums: at N = 2 n - 2 the last one came twice
     auto lin = [&](int j) { return j >= nl ? 0.0 : (N[d] == 2 * nl - 2 && j == nl - 1) ? 0.5 * R[j] : R[j]; };
-    for (int m = 0; m < nkeep; ++m) *SkTot++ = (lin(m) + lin(nl - m)) / (stdDev * stdDev * (double)n);
+    for (int m = 0; m < nkeep; ++m) *SkTot++ = (lin(m) + lin(nl - m)) / (sd * sd * (double)n);
   }
   return SCARL_OK;
 }
