@@ -3375,9 +3375,18 @@ int scarl_rebuild_sk(scarl_ctx* ctx, const void* field, int dtype, const int L[3
   }
   const void* tw[3];
   for (int d = 0; d < 3; ++d) RC(twiddles(ctx, N[d], 8, &tw[d]));
-  RC(ensure(ctx, ctx->part, pbytes));
   RC(ensure(ctx, ctx->t2, ((size_t)nmax + nw) * 8));
   RC(ensure(ctx, ctx->tabs, nw * 8));
+  // fewer blocks (which walk more lines each) where the budget has no room for a
+  // row of partial sums of every one
+  for (int rc; (rc = ensure(ctx, ctx->part, pbytes)) != SCARL_OK;) {
+    if (rc != SCARL_ENOMEM || (nb[0] == 1 && nb[1] == 1 && nb[2] == 1)) return rc;
+    pbytes = 0;
+    for (int d = 0; d < 3; ++d) {
+      nb[d] = (nb[d] + 1) / 2;
+      pbytes = std::max(pbytes, (size_t)nb[d] * N[d] * 8);
+    }
+  }
   double* bins = (double*)ctx->t2.p;
   double* S = bins + nmax;
   void* hp;
