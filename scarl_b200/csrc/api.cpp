@@ -38,6 +38,7 @@ struct Buf {
 
 // A pinned host buffer and the event of its last upload.
 constexpr int kPinSlots = 8;
+constexpr size_t kPinSmall = (size_t)1 << 20;
 struct PinSlot {
   void* p = nullptr;
   size_t n = 0;
@@ -171,6 +172,8 @@ struct scarl_ctx {
   Buf mom;     // FP64 partial pairs of the streamed moments (pass 3) and their sum
   int wait_test = 0;  // test hook of the bounded tensor-core waits
   PinSlot pins[kPinSlots];  // pinned staging of small uploads, used in turn
+  PinSlot pin_large;        // and of larger ones
+  PinSlot* pin_last = nullptr;
   int pin_cur = 0;
   // device -> pinned host copies of finished z slabs, overlapped with the
   // generation of the remaining tiles
@@ -302,13 +305,15 @@ bool is_pinned_host(const void* p) {
   return a.type == cudaMemoryTypeHost;
 }
 
-// Pinned host staging for small tables: the next of kPinSlots buffers, once the
-// upload that last used it is done.  (With one buffer each upload waited for
+// Pinned host staging: the next of kPinSlots buffers, once the upload that last
+// used it is done; one buffer of its own for what exceeds kPinSmall (large tables,
+// blocks on their way to a file), so that the context pins kPinSlots kPinSmall bytes
+// beside the largest request.  (With one buffer for all, each upload waited for
 // the previous one, which sits in the stream behind the previous call's kernels:
 // the host never ran ahead of the GPU.)
 int pinned(scarl_ctx* ctx, size_t bytes, void** out) {
-  ctx->pin_cur = (ctx->pin_cur + 1) % kPinSlots;
-  PinSlot& b = ctx->pins[ctx->pin_cur];
+  if (bytes <= kPinSmall) ctx->pin_cur = (ctx->pin_cur + 1) % kPinSlots;
+  PinSlot& b = bytes <= kPinSmall ? ctx->pins[ctx->pin_cur] : ctx->pin_large;
   if (b.ev) CK(cudaEventSynchronize(b.ev));
   if (b.n < bytes) {
     if (b.p) cudaFreeHost(b.p);
@@ -317,13 +322,14 @@ int pinned(scarl_ctx* ctx, size_t bytes, void** out) {
     CK(cudaMallocHost(&b.p, bytes));
     b.n = bytes;
   }
+  ctx->pin_last = &b;
   *out = b.p;
   return SCARL_OK;
 }
 
 // Uploads the buffer that the last call of pinned returned.
 int upload_pinned(scarl_ctx* ctx, void* dst, size_t bytes) {
-  PinSlot& b = ctx->pins[ctx->pin_cur];
+  PinSlot& b = *ctx->pin_last;
   CK(cudaMemcpyAsync(dst, b.p, bytes, cudaMemcpyHostToDevice, ctx->stream));
   ctx->h2d += bytes;
   if (!b.ev) CK(cudaEventCreateWithFlags(&b.ev, cudaEventDisableTiming));
@@ -1760,10 +1766,12 @@ int scarl_ctx_destroy(scarl_ctx* ctx) {
   ens_free(ctx);
   for (Buf* b : {&ctx->mlp_p, &ctx->mlp_m, &ctx->mlp_v, &ctx->mlp_g, &ctx->mlp_wb}) release(ctx, *b);
   for (cudaEvent_t e : ctx->pool) cudaEventDestroy(e);
-  for (PinSlot& b : ctx->pins) {
+  auto unpin = [](PinSlot& b) {
     if (b.ev) cudaEventDestroy(b.ev);
     if (b.p) cudaFreeHost(b.p);
-  }
+  };
+  for (PinSlot& b : ctx->pins) unpin(b);
+  unpin(ctx->pin_large);
   for (cudaEvent_t e : ctx->slab_ev) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->ring_ev)
     if (e) cudaEventDestroy(e);
