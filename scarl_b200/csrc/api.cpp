@@ -1371,7 +1371,13 @@ int dct_table(scarl_ctx* ctx, int N, int K, const double** tab, const double** r
   if (!*roots) {
     RC(ensure(ctx, r, raw));
     std::vector<double> c(4 * (size_t)N);
-    for (int64_t m = 0; m < 4 * (int64_t)N; ++m) c[m] = std::cos(M_PI * (double)m / (2.0 * (double)N));
+    // cos(pi m / 2N) rounded once: the first quarter turn, the others by symmetry
+    const int64_t n1 = N, n2 = 2 * (int64_t)N;
+    const long double step = 3.14159265358979323846264338327950288L / (long double)n2;
+    for (int64_t m = 0; m < n1; ++m) c[m] = (double)cosl(step * (long double)m);
+    c[n1] = 0.0;
+    for (int64_t m = n1 + 1; m < n2; ++m) c[m] = -c[n2 - m];
+    for (int64_t m = 0; m < n2; ++m) c[n2 + m] = -c[m];
     const int rc = put_table(ctx, r.p, c.data(), raw);
     if (rc != SCARL_OK) {
       release(ctx, r);
