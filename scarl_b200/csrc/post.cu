@@ -19,22 +19,23 @@ static inline unsigned grid_for(int64_t n, int threads, int cap = 148 * 32) {
 
 struct PouAxes { BlendAxis ax[3]; };
 
-// A warp a row of x (the row's y and z found once, with 32-bit arithmetic): f *=
-// sqrt(w), the factors multiplied in the reference's order.  A factor of
-// exactly 1, the inside of the tile, leaves the value as it is: neither read
-// nor written.  Bound by launch latency at the sizes of the drop-in steps (95 x
-// 78 x 83 FP64 points: 12.8 -> 11.4 us between two timing events, of which an
-// empty kernel takes about 5), against a thread a point with 64-bit divisions.
-constexpr int kRowsPerBlock = 8;
-template <typename T>
-__global__ void __launch_bounds__(32 * kRowsPerBlock) k_apply_pou(T* __restrict__ f, int Nx, int Ny, int nrows,
+// A warp a row of x (the row's y and z found once, with 32-bit arithmetic where
+// the rows and the walk's last step allow it: I): f *= sqrt(w), the factors
+// multiplied in the reference's order.  A factor of exactly 1, the inside of the
+// tile, leaves the value as it is: neither read nor written.  Bound by launch
+// latency at the sizes of the drop-in steps (95 x 78 x 83 FP64 points: 12.8 -> 11.4
+// us between two timing events, of which an empty kernel takes about 5), against a
+// thread a point with 64-bit divisions.
+constexpr int kRowsPerBlock = 8, kRowBlocks = 148 * 64;
+template <typename T, typename I>
+__global__ void __launch_bounds__(32 * kRowsPerBlock) k_apply_pou(T* __restrict__ f, int Nx, int Ny, I nrows,
                                                                   const PouAxes p) {
   const int lane = threadIdx.x & 31;
-  for (int row = blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5); row < nrows; row += gridDim.x * kRowsPerBlock) {
-    const int z = row / Ny, y = row - z * Ny;
+  for (I row = (I)(blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5)); row < nrows; row += (I)(gridDim.x * kRowsPerBlock)) {
+    const int z = (int)(row / Ny), y = (int)(row - (I)z * Ny);
     const double ly = p.ax[1].lo[y], lz = p.ax[2].lo[z], hy = p.ax[1].hi[y], hz = p.ax[2].hi[z];
     T* r = f + (int64_t)row * Nx;
-    for (int x = lane; x < Nx; x += 32) {
+    for (unsigned x = lane; x < (unsigned)Nx; x += 32) {
       double w = p.ax[0].lo[x];
       w = __dmul_rn(w, ly);
       w = __dmul_rn(w, lz);
@@ -46,14 +47,21 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) k_apply_pou(T* __restrict_
   }
 }
 
+template <typename T>
+static void apply_pou(unsigned g, T* field, const int Np[3], int64_t rows, const PouAxes& p, cudaStream_t s) {
+  if (rows <= 2147483647LL - kRowBlocks * kRowsPerBlock)
+    k_apply_pou<T, int><<<g, 32 * kRowsPerBlock, 0, s>>>(field, Np[0], Np[1], (int)rows, p);
+  else
+    k_apply_pou<T, int64_t><<<g, 32 * kRowsPerBlock, 0, s>>>(field, Np[0], Np[1], rows, p);
+}
+
 cudaError_t launch_apply_pou(int dt, void* field, const int Np[3], const BlendAxis ax[3],
                              cudaStream_t s) {
   PouAxes p{{ax[0], ax[1], ax[2]}};
   const int64_t rows = (int64_t)Np[1] * Np[2];
-  if (rows > 2147483647LL) return cudaErrorInvalidValue;
-  const unsigned g = grid_for(rows, kRowsPerBlock, 148 * 64);
-  if (dt == 8) k_apply_pou<double><<<g, 32 * kRowsPerBlock, 0, s>>>((double*)field, Np[0], Np[1], (int)rows, p);
-  else k_apply_pou<float><<<g, 32 * kRowsPerBlock, 0, s>>>((float*)field, Np[0], Np[1], (int)rows, p);
+  const unsigned g = grid_for(rows, kRowsPerBlock, kRowBlocks);
+  if (dt == 8) apply_pou(g, (double*)field, Np, rows, p, s);
+  else apply_pou(g, (float*)field, Np, rows, p, s);
   return cudaGetLastError();
 }
 
@@ -69,7 +77,8 @@ struct OvlArgs { int Np[3], No[3], T[3]; };
 __global__ void __launch_bounds__(32 * kRowsPerBlock) k_add_overlap(const double* __restrict__ in, double* __restrict__ out,
                                                                     const OvlArgs a, int64_t nrows) {
   const int lane = threadIdx.x & 31;
-  const int Nx = a.Np[0], Ny = a.Np[1], Nz = a.Np[2], rows = Ny * Nz;
+  const int Nx = a.Np[0], Ny = a.Np[1], Nz = a.Np[2];
+  const int64_t rows = (int64_t)Ny * Nz;
   // direction s along axis d reaches coordinate c of a tile at position pos:
   // s = 1 the low side, -1 the high side, 0 the tile's own extent; degenerate
   // regions (one point) never
@@ -80,8 +89,9 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) k_add_overlap(const double
   };
   for (int64_t q = (int64_t)blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5); q < nrows;
        q += (int64_t)gridDim.x * kRowsPerBlock) {
-    const int r = (int)(q / rows), yz = (int)(q - (int64_t)r * rows);
-    const int z = yz / Ny, y = yz - z * Ny;
+    const int r = (int)(q / rows);
+    const int64_t yz = q - r * rows;
+    const int z = (int)(yz / Ny), y = (int)(yz - (int64_t)z * Ny);
     const int pz = r / (a.T[0] * a.T[1]), rest = r - pz * a.T[0] * a.T[1], py = rest / a.T[0], px = rest - py * a.T[0];
     unsigned m = 0;  // bit 3 (kk + 1) + (jj + 1)
     for (int kk = -1; kk <= 1; ++kk)
@@ -89,7 +99,7 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) k_add_overlap(const double
         if (reaches(2, kk, z, pz) && reaches(1, jj, y, py)) m |= 1u << (3 * (kk + 1) + jj + 1);
     if (!m) continue;
     const int dx = Nx - a.No[0], dy = Ny - a.No[1], dz = Nz - a.No[2];
-    for (int x = lane; x < Nx; x += 32) {
+    for (int64_t x = lane; x < Nx; x += 32) {
       const bool xl = reaches(0, 1, x, px), xh = reaches(0, -1, x, px), x0 = Nx > 1;
       if (!xl && !xh && (m & ~(1u << 4)) == 0) continue;
       if (!xl && !xh && !x0) continue;
@@ -114,8 +124,7 @@ cudaError_t launch_add_overlap(const double* in, double* out, const int Np[3],
   OvlArgs a;
   for (int d = 0; d < 3; ++d) { a.Np[d] = Np[d]; a.No[d] = Np_ovlp[d]; a.T[d] = topo[d]; }
   const int64_t rows = (int64_t)Np[1] * Np[2] * topo[0] * topo[1] * topo[2];
-  if ((int64_t)Np[1] * Np[2] > 2147483647LL) return cudaErrorInvalidValue;
-  k_add_overlap<<<grid_for(rows, kRowsPerBlock, 148 * 64), 32 * kRowsPerBlock, 0, s>>>(in, out, a, rows);
+  k_add_overlap<<<grid_for(rows, kRowsPerBlock, kRowBlocks), 32 * kRowsPerBlock, 0, s>>>(in, out, a, rows);
   return cudaGetLastError();
 }
 
