@@ -145,13 +145,14 @@ class HostPool {
 constexpr int kRingSlots = 4;
 constexpr size_t kRingChunk = (size_t)32 << 20;
 constexpr size_t kRingMin = (size_t)8 << 20;
-// literal DCT tiles generated and held together up to this many bytes: few
-// launches over all of them, the tiles and the y step's output staying in the
-// 126 MB L2 for the gather.  8 tiles of 23^3, 66^3, 96^3 (0.8, 18, 57 MB): 58, 92,
-// 181 us a sample against 203, 271, 319 tile by tile; past the L2 the gain fades
-// (83 MB 84 against 115) and ends (252 MB 254 against 244, 941 MB 869 against 583),
-// where one tile fills the GPU and saves the tiles' round trip through memory
-constexpr size_t kDctBatch = (size_t)64 << 20;
+// literal DCT tiles up to the first size each and the second together are generated
+// in few launches over all of them and blended by one gather; larger ones, which
+// fill the GPU by themselves, one after the other, each saving the round trip of
+// its tile through memory.  Together against one by one, us a sample: 8 tiles of
+// 23^3, 66^3, 96^3, 112^3, 128^3, 160^3 (0.1 .. 31 MB each) 54 / 191, 97 / 262,
+// 190 / 321, 296 / 379, 400 / 394, 918 / 784; 27 of 100^3 (206 MB) 689 / 1251; 4
+// of 140^3 342 / 359; 2 of 160^3 (62 MB) 237 / 195, of 200^3 444 / 318
+constexpr size_t kDctTile = (size_t)16 << 20, kDctBatch = (size_t)256 << 20;
 // a cosine matrix is kept up to the first size (lengths to 8192 over half the
 // inputs, 5793 over all), all of them together up to the second; longer axes form
 // their cosines in the kernel (8300 points along x / y / z by 64 x 64: 2.6 / 4.9 /
@@ -2876,11 +2877,12 @@ int scarl_generate_sample(scarl_ctx* ctx, const scarl_sample* s, const scarl_gen
   const void* phi_all = nullptr;
   if (gen == SCARL_GEN_DCT && o.phiK)
     RC(in_dev(ctx, ctx->stage_in, o.phiK, nk * lay.nb_tiles * 8, &phi_all));
-  // literal tiles that fit kDctBatch bytes together: one launch per step over all
-  // of them, then one gather of the blended field.  Larger ones, and those whose
-  // buffers together find no room, one after the other, each blended by its z
-  // transform's output stage.
-  bool dct_batch = gen == SCARL_GEN_DCT && lay.nb_tiles > 1 && ntile * 8 * lay.nb_tiles <= kDctBatch;
+  // small literal tiles (kDctTile, kDctBatch): one launch per step over all of them,
+  // then one gather of the blended field.  Larger ones, and those whose buffers
+  // together find no room, one after the other, each blended by its z transform's
+  // output stage.
+  bool dct_batch = gen == SCARL_GEN_DCT && lay.nb_tiles > 1 && ntile * 8 <= kDctTile &&
+                   ntile * 8 * lay.nb_tiles <= kDctBatch;
   if (dct_batch) {
     std::vector<double> xr((size_t)3 * lay.nb_tiles);
     for (int q = 0; q < lay.nb_tiles; ++q) {
