@@ -1,7 +1,8 @@
-// epilogue.cuh -- per-point output stage of the C2R pass: plain crop, or partition-of-unity blend into the global
-// field (SRC_F/main_ScaRL.f90:1216-1301 weights, 984-1210 overlap sum,
-// write_output.f90:373-431 assembly) with the marginal transform
-// (SRC_F/main_ScaRL.f90:1355-1395) applied by the tile that finishes a point.
+// epilogue.cuh -- per-point output stage of the C2R pass: plain crop, or
+// partition-of-unity blend into the global field (SRC_F/main_ScaRL.f90:1216-1301
+// weights, 984-1210 overlap sum, write_output.f90:373-431 assembly) with the
+// marginal transform (SRC_F/main_ScaRL.f90:1355-1395) applied by the tile that
+// finishes a point.
 #pragma once
 
 #include "scarl_common.cuh"
