@@ -104,8 +104,8 @@ __device__ __forceinline__ int rsq_order(double expo) {
 // the first DFT stage they were some 1000 instructions with a power and two
 // branches each, and the kernel waited on instruction fetches (2.2 of 10.8
 // stalled warps per issue).  As a loop, with 32-bit counters and flushed hardware
-// functions: 348 -> 284 us on a 512^3 grid (201 planes kept), FP64 122 -> 100 us
-// on 256 x 224 x 256.
+// functions: 348 -> 293 us on a 512^3 grid (201 planes kept), FP64 122 -> 90 us on
+// 256 x 224 x 256.
 // ---------------------------------------------------------------------------
 template <typename T, class Kz, class Put>
 __device__ __forceinline__ void synth_line(const GenArgs& a, int kx, int ky, Kz kzof, int nd, int N, Put put) {

@@ -96,12 +96,12 @@ int gen_pass3_partials(int dt, int v, const GenArgs& a) {
 // of every variant over lengths 32 .. 2048 on grids of 12 - 24 M modes, crop mode.
 //
 // Passes 1 and 2: the two-stage kernels for lengths m 2^a (m = 3, 5, 7), whose
-// engine plans take four or five stages (FP32 pass 1 / pass 2, us: 224 69.8 /
-// 25.1 against 90.5 / 33.2, 384 66 / 24 against 70 / 30, 448 81 / 27 against 92 /
-// 35; FP64 224 98 / 27 against 138 / 33), and for short powers of two.  Longer
-// powers of two keep two or three engine stages, with 32 values a thread in the
-// FP32 pass 2 from 512 on (33.3 against 36.9, 1024 39.5 against 43.5) and eight in
-// the FP64 pass 1 (256 101 against 108, 1024 122 against 155).
+// engine plans take four or five stages (FP32 pass 1 / pass 2, us: 224 71 / 25
+// against 89 / 33, 384 66 / 23 against 70 / 31, 448 82 / 29 against 91 / 35; FP64
+// 224 92 / 27 against 127 / 33), and for short powers of two.  Longer powers of two
+// keep two or three engine stages, with 32 values a thread in the FP32 pass 2 from
+// 512 on (31.8 against 35.4, 1024 36.9 against 45.6) and eight in the FP64 pass 1
+// (256 94.5 against 98.7, 1024 118 against 140).
 // Pass 3: the two-stage kernel where it serves the half length (FP32 224 / 256 /
 // 384 / 512: 47 / 45 / 48 / 65 against 58 / 62 / 66 / 72 for the best other; FP64
 // 112 / 224 / 256: 46 / 45 / 46 against 80 / 117 / 72), except FP32 lines of 64 and
